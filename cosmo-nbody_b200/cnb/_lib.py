@@ -76,6 +76,8 @@ SIGNATURES = {
     "cnb_build_top_tree_cache": (_int, [_p, _p, _p, _p, _i32, _p]),
     "cnb_compute_forces": (_int, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _d, _d, _d, _d, _p, _i64,
                                   _i64, _i64, _int, _p, _p]),
+    "cnb_compute_forces_table": (_int, [_p, _p, _p, _p, _p, _d, _d, _d, _d, _p, _i64, _i64, _i64,
+                                        _int, _p, _p]),
     "cnb_integrate": (_int, [_p, _p, _p, _p, _p, _p, _p, _i64, _d, _d, _d, _p]),
     "cnb_render_density": (_int, [_p, _p, _p, _p, _p, _i64, _int, _int, _p]),
     "cnb_pack_nodes": (_int, [_p, _p, _p, _p, _p, _p, _i64, _p]),

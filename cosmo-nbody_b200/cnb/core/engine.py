@@ -93,6 +93,9 @@ class SimulationEngine:
         if self.force_mode == "grouped":
             self.set_super_bodies(int(getattr(config, "SUPER_BODIES", 0)))
         self.precision = _lib.PREC_F64 if getattr(config, "PRECISION", "f32") == "f64" else _lib.PREC_F32
+        # reference mode: the node records the per-body walk reads
+        self.ref_table = (torch.empty((4, self.tree_manager.n_nodes, 4), dtype=torch.float32,
+                                      device=state.device) if self.force_mode == "reference" else None)
         self.stage_events = None
         self.nvtx = False          # NVTX ranges around the step's stages (for nsys / ncu timelines)
         self._nvtx_open = False
@@ -180,11 +183,14 @@ class SimulationEngine:
                       self.bodies_per_lane, self.block_warps, float(cfg.G), float(cfg.SOFTENING),
                       float(cfg.BOX_SIZE), self.slab_mass, self.stats.data_ptr(), status, st)
         else:
-            _lib.call("cnb_compute_forces", px.data_ptr(), py.data_ptr(), pz.data_ptr(),
-                      tm.child.data_ptr(), tm.mass.data_ptr(), tm.com.data_ptr(),
-                      tm.aabb_min.data_ptr(), tm.aabb_max.data_ptr(), s.force.data_ptr(),
-                      float(cfg.THETA), float(cfg.G), float(cfg.SOFTENING), float(cfg.BOX_SIZE),
-                      tm.root_idx.data_ptr(), 0, s.n, s.n, self.precision, status, st)
+            # the nodes once as 32-byte records, then the walk over them
+            _lib.call("cnb_pack_nodes", tm.mass.data_ptr(), tm.com.data_ptr(), tm.aabb_min.data_ptr(),
+                      tm.aabb_max.data_ptr(), tm.child.data_ptr(), self.ref_table.data_ptr(),
+                      tm.n_nodes, st)
+            _lib.call("cnb_compute_forces_table", px.data_ptr(), py.data_ptr(), pz.data_ptr(),
+                      self.ref_table.data_ptr(), s.force.data_ptr(), float(cfg.THETA), float(cfg.G),
+                      float(cfg.SOFTENING), float(cfg.BOX_SIZE), tm.root_idx.data_ptr(), 0, s.n, s.n,
+                      self.precision, status, st)
 
     _NEXT_STAGE = {"start": "sort", "sort": "tree", "tree": "forces"}
 

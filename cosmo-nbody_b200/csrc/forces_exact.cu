@@ -52,8 +52,6 @@
 
 namespace cnb {
 
-constexpr float kCutLo = 0.99999e-7f, kCutHi = 1.00001e-7f;  // float64 band around the cut
-
 // The two node stacks of a warp share one region of XW words: entries
 // reached by the whole bucket (one word, the node) grow up from word 0,
 // entries reached by part of it (three words: node, mask low, mask high)
@@ -98,21 +96,6 @@ __device__ __forceinline__ float minus_image(float d) {
 __device__ __forceinline__ float2 minus_image2(float2 d) {
     const float2 rc = dup2(12582912.f), nrc = dup2(-12582912.f);
     return __ffma2_rn(__fadd2_rn(__fadd2_rn(d, rc), nrc), dup2(-1.f), d);
-}
-
-// The reference's test for one body, sx^2 < theta^2 d^2, in float64: called
-// only when the float32 d^2 lies within the margin band of s^2 / theta^2.
-__device__ __noinline__ bool ref_accepts_f64(float s, double th2d, float dx, float dy, float dz) {
-    const double d2d = (double)dx * dx + (double)dy * dy + (double)dz * dz;
-    return (double)s * (double)s < th2d * d2d;
-}
-
-// The reference's cut d^2 > 1e-7 (float64), float32 outside a narrow band.
-__device__ __forceinline__ bool ref_outside_cut(float dx, float dy, float dz, float d2) {
-    if (d2 > kCutHi) return true;
-    if (d2 < kCutLo) return false;
-    const double d2d = (double)dx * dx + (double)dy * dy + (double)dz * dz;
-    return d2d > 1e-7;
 }
 
 // Entry j of a list as the two packed float4 (x, x, y, y), (z, z, m, m) of the
@@ -730,7 +713,15 @@ static int launch_exact_shape(GroupedParams &P, cudaStream_t st) {
 
 static int g_test_spill_every = 0;  // cnb_exact_test_spill
 
+// Systems of at most this many bodies take the walk by groups (forces_ref.cu):
+// their few hundred buckets leave most warps of the chip idle while each is a
+// serial walk of some 90 000 instructions.  Measured, theta 0.5 (us, buckets
+// against groups): 4 096 bodies 172 / 36, 32 768 412 / 141, 65 536 482 / 276,
+// 131 072 495 / 529.
+constexpr int64_t kWalkBodies = 98304;
+
 int launch_exact(GroupedParams &P, int bodies_per_lane, int block_warps, cudaStream_t st) {
+    if (P.n <= kWalkBodies && !P.box_roots && !P.theta_per_bucket) return launch_exact_walk(P, st);
     P.test_spill_every = g_test_spill_every;
     switch (bodies_per_lane * 16 + block_warps) {
         case 16 + 2: return launch_exact_shape<1, 2>(P, st);

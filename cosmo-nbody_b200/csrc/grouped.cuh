@@ -78,6 +78,23 @@ constexpr float kCutGuard = 2e-7f;
 constexpr float kBoxSlack = 1e-6f;
 constexpr float kRelMargin = 4e-6f;
 
+constexpr float kCutLo = 0.99999e-7f, kCutHi = 1.00001e-7f;  // float64 band around the cut
+
+// The reference's test for one body, sx^2 < theta^2 d^2, in float64: called
+// only when the float32 d^2 lies within the margin band of s^2 / theta^2.
+static __device__ __noinline__ bool ref_accepts_f64(float s, double th2d, float dx, float dy, float dz) {
+    const double d2d = (double)dx * dx + (double)dy * dy + (double)dz * dz;
+    return (double)s * (double)s < th2d * d2d;
+}
+
+// The reference's cut d^2 > 1e-7 (float64), float32 outside a narrow band.
+__device__ __forceinline__ bool ref_outside_cut(float dx, float dy, float dz, float d2) {
+    if (d2 > kCutHi) return true;
+    if (d2 < kCutLo) return false;
+    const double d2d = (double)dx * dx + (double)dy * dy + (double)dz * dz;
+    return d2d > 1e-7;
+}
+
 // Applies cnt list entries (x, y, z, mass) to the lane's BPL bodies.  WRAP:
 // the entries' image may differ between the bucket's bodies, so every pair
 // takes its own minimum image.  CUT: apply the reference's d^2 > 1e-7 cut.
@@ -222,5 +239,8 @@ __device__ __forceinline__ void apply_entries(const float4 *list, int cnt, const
 // forces_exact.cu: the grouped traversal with the reference's per-body
 // opening decisions (CNB_MAC_REF_X); P.ws[1] must be zero.
 int launch_exact(GroupedParams &P, int bodies_per_lane, int block_warps, cudaStream_t st);
+
+// forces_ref.cu: the same decisions and forces by groups of consecutive bodies, for small systems.
+int launch_exact_walk(const GroupedParams &P, cudaStream_t st);
 
 }  // namespace cnb

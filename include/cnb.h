@@ -237,6 +237,16 @@ int cnb_compute_forces(const float *px, const float *py, const float *pz,
                        double G, double soft, double box, const int32_t *root_idx, int64_t off,
                        int64_t count, int64_t n, int precision, int32_t *status, void *stream);
 
+/* cnb_compute_forces reading the tree from a node table (cnb_pack_nodes of the
+ * same arrays: the same values, 32 bytes a node) instead of the reference's
+ * arrays.  The same nodes and arithmetic for every target; faster for many
+ * targets, where one pass over the nodes to pack them is cheap. */
+int cnb_compute_forces_table(const float *px, const float *py, const float *pz,
+                             const float *node_table, float *force, double theta, double G,
+                             double soft, double box, const int32_t *root_idx, int64_t off,
+                             int64_t count, int64_t n, int precision, int32_t *status,
+                             void *stream);
+
 /* src/kernels/physics_kernels.py:155-203 integrate(pos_x, pos_y, pos_z, vel_x, vel_y,
  * vel_z, force, a, H, dt). */
 int cnb_integrate(float *px, float *py, float *pz, float *vx, float *vy, float *vz,
