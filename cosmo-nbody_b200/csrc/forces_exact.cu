@@ -36,10 +36,14 @@
 // the entry's mask); every other accepted entry keeps the node's raw CoM and
 // is applied with the per-pair minimum image, the cut and its mask.
 // Per-body items carry the band [lo, hi] around s^2 / theta^2 inside which
-// the float32 d^2 cannot decide, and flags for the per-pair image and the
-// cut, so the common item is a handful of packed operations per body pair;
-// lane j keeps item j's mask of opening bodies and the children of a round's
-// items are pushed together after them.
+// the float32 d^2 cannot decide.  Most are simple (87 % at 128^3): one image
+// for every body, out of the cut's reach, and a CoM that shifts to that image
+// exactly, so a round applies them first, without image, cut or flags; the
+// others follow with the per-pair form.  Each lane keeps the node it
+// classified, the mask of the bodies that accept it comes back to it, and the
+// children of a round's items are pushed together after them.  Measured
+// against one loop over flagged items (128^3, theta 0.5, 64-body buckets,
+// two-level): 4.98 -> 4.74 ms; 32-body buckets, one level: 7.25 -> 6.72 ms.
 //
 // The node stacks live in shared memory (see kXWords); a bucket that would
 // outgrow them in the main pass is walked again by a second launch with a
@@ -124,6 +128,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
                                              const float (&z)[BPL], float soft2, float (&ax)[BPL],
                                              float (&ay)[BPL], float (&az)[BPL]) {
     const float cut = soft2 + 1e-7f;
+    const uint32_t lane_bit = 1u << lane;
     if constexpr (BPL == 2) {
         const float2 nx = make_float2(-x[0], -x[1]), ny = make_float2(-y[0], -y[1]),
                      nz = make_float2(-z[0], -z[1]);
@@ -149,7 +154,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
                     dz[u] = minus_image2(dz[u]);
                 }
                 q[u] = __ffma2_rn(dx[u], dx[u], __ffma2_rn(dy[u], dy[u], __ffma2_rn(dz[u], dz[u], s2)));
-                const bool u0 = (mk.x >> lane) & 1u, u1 = (mk.y >> lane) & 1u;
+                const bool u0 = (mk.x & lane_bit) != 0u, u1 = (mk.y & lane_bit) != 0u;
                 w[u] = make_float2(u0 && (!WRAP_CUT || q[u].x > cut) ? b.z : 0.f,
                                    u1 && (!WRAP_CUT || q[u].y > cut) ? b.w : 0.f);
             }
@@ -175,7 +180,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
                 dz = minus_image2(dz);
             }
             const float2 q = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, s2)));
-            const bool u0 = (mk.x >> lane) & 1u, u1 = (mk.y >> lane) & 1u;
+            const bool u0 = (mk.x & lane_bit) != 0u, u1 = (mk.y & lane_bit) != 0u;
             const float2 w = make_float2(u0 && (!WRAP_CUT || q.x > cut) ? b.z : 0.f,
                                          u1 && (!WRAP_CUT || q.y > cut) ? b.w : 0.f);
             const float2 r = make_float2(rsqrtf(q.x), rsqrtf(q.y));
@@ -191,7 +196,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
 #pragma unroll 4
         for (int j = 0; j < cnt; ++j) {
             const float4 e = list[j];
-            const bool u = (masks[j].x >> lane) & 1u;
+            const bool u = (masks[j].x & lane_bit) != 0u;
 #pragma unroll
             for (int b = 0; b < BPL; ++b) {
                 float dx = e.x - x[b], dy = e.y - y[b], dz = e.z - z[b];
@@ -278,6 +283,73 @@ __device__ __forceinline__ void per_body_item(float4 I, float4 J, uint32_t m0, u
             ay[b] = fmaf(f, dy, ay[b]);
             az[b] = fmaf(f, dz, az[b]);
         }
+    }
+}
+
+// The rare outcome of a simple item: d^2 within the band around s^2 / theta^2.
+// The reference's own float32 differences (from the node's record, not the
+// shifted CoM of the item) and its float64 test.
+static __device__ __noinline__ bool accepts_f64(const float4 *__restrict__ rec, int node, float box,
+                                                double th2d, float x, float y, float z) {
+    const float4 A = __ldg(rec + 2 * (int64_t)node);
+    const float sx = __ldg(rec + 2 * (int64_t)node + 1).x;
+    return ref_accepts_f64(sx > 0.5f * box ? box : sx, th2d, minus_image(A.x - x),
+                           minus_image(A.y - y), minus_image(A.z - z));
+}
+
+// One simple item: its CoM at the one image every body of the bucket sees,
+// out of the cut's reach.  For two bodies per lane I = (x, x, y, y), J = (z,
+// z, m, node), K = (lo, hi, mask); for one I = (x, y, z, m), J.w = node.
+// [lo, hi] is the band around s^2 / theta^2 where the float32 d^2 does not
+// decide.  Adds the force of the bodies that accept the node and returns them
+// (b0, b1): what is left of the mask opens it.
+template <int BPL>
+__device__ __forceinline__ uint2 simple_item(float4 I, float4 J, float4 K, uint32_t lane_bit,
+                                             const float4 *rec, float box, double th2d, float soft2,
+                                             const float (&x)[BPL], const float (&y)[BPL],
+                                             const float (&z)[BPL], float (&ax)[BPL],
+                                             float (&ay)[BPL], float (&az)[BPL]) {
+    if constexpr (BPL == 2) {
+        const float2 dx = __fadd2_rn(make_float2(I.x, I.y), make_float2(-x[0], -x[1]));
+        const float2 dy = __fadd2_rn(make_float2(I.z, I.w), make_float2(-y[0], -y[1]));
+        const float2 dz = __fadd2_rn(make_float2(J.x, J.y), make_float2(-z[0], -z[1]));
+        const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        bool p0 = d2.x > K.y, p1 = d2.y > K.y;
+        if ((!p0 && !(d2.x < K.x)) || (!p1 && !(d2.y < K.x))) {
+            const int node = __float_as_int(J.w);
+            if (!p0 && !(d2.x < K.x)) p0 = accepts_f64(rec, node, box, th2d, x[0], y[0], z[0]);
+            if (!p1 && !(d2.y < K.x)) p1 = accepts_f64(rec, node, box, th2d, x[1], y[1], z[1]);
+        }
+        p0 = p0 && (__float_as_uint(K.z) & lane_bit) != 0u;
+        p1 = p1 && (__float_as_uint(K.w) & lane_bit) != 0u;
+        const uint2 acc = make_uint2(__ballot_sync(0xffffffffu, p0), __ballot_sync(0xffffffffu, p1));
+        // an item every reaching body opens adds no force (a third of them)
+        if ((acc.x | acc.y) == 0u) return acc;
+        const float2 q = __fadd2_rn(d2, dup2(soft2));
+        const float2 r = make_float2(rsqrtf(q.x), rsqrtf(q.y));
+        const float2 w = make_float2(p0 ? J.z : 0.f, p1 ? J.z : 0.f);
+        const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, r), r), r);
+        const float2 fx = __ffma2_rn(f, dx, make_float2(ax[0], ax[1]));
+        const float2 fy = __ffma2_rn(f, dy, make_float2(ay[0], ay[1]));
+        const float2 fz = __ffma2_rn(f, dz, make_float2(az[0], az[1]));
+        ax[0] = fx.x; ax[1] = fx.y;
+        ay[0] = fy.x; ay[1] = fy.y;
+        az[0] = fz.x; az[1] = fz.y;
+        return acc;
+    } else {
+        const float dx = I.x - x[0], dy = I.y - y[0], dz = I.z - z[0];
+        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        bool p = d2 > K.y;
+        if (!p && !(d2 < K.x)) p = accepts_f64(rec, __float_as_int(J.w), box, th2d, x[0], y[0], z[0]);
+        p = p && (__float_as_uint(K.z) & lane_bit) != 0u;
+        const uint32_t acc = __ballot_sync(0xffffffffu, p);
+        if (acc == 0u) return make_uint2(0u, 0u);
+        const float r = rsqrtf(d2 + soft2);
+        const float f = p ? I.w * r * r * r : 0.f;
+        ax[0] = fmaf(f, dx, ax[0]);
+        ay[0] = fmaf(f, dy, ay[0]);
+        az[0] = fmaf(f, dz, az[0]);
+        return make_uint2(acc, 0u);
     }
 }
 
@@ -479,7 +551,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
             const bool whole = mk.x == fm.x && mk.y == fm.y;
             // 1: accepted by every body of the mask, 2: opened by every one, 3: per body
             int cls = 0;
-            bool one_image = false, zero_image = false, near_box = false;
+            bool one_image = false, simple = false, shifted = false, near_box = false;
             float4 A = make_float4(0.f, 0.f, 0.f, 0.f), E = A;
             float s = 0.f;
             int32_t c0 = -1, c1 = -1;
@@ -509,8 +581,11 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                     }
                     near_box = d2min <= kCutGuard;
                     one_image = adx < wlx && ady < wly && adz < wlz;
-                    zero_image = one_image && sx_ == 0.f && sy_ == 0.f && sz_ == 0.f;
+                    shifted = sx_ != 0.f || sy_ != 0.f || sz_ != 0.f;
                     E = make_float4(A.x - sx_, A.y - sy_, A.z - sz_, A.w);
+                    // a per-body item takes the shifted CoM when the shift is exact in float32
+                    simple = one_image && !near_box && E.x + sx_ == A.x && E.y + sy_ == A.y &&
+                             E.z + sz_ == A.z;
                 }
             }
             b_tests += (node >= 0);
@@ -522,7 +597,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
             const uint32_t m_x = __ballot_sync(0xffffffffu, to_x);
             const uint32_t m_ow = __ballot_sync(0xffffffffu, cls == 2 && whole);
             const uint32_t m_op = __ballot_sync(0xffffffffu, cls == 2 && !whole);
-            const uint32_t m_pb = __ballot_sync(0xffffffffu, cls == 3);
+            const uint32_t m_ps = __ballot_sync(0xffffffffu, cls == 3 && simple);
+            const uint32_t m_pg = __ballot_sync(0xffffffffu, cls == 3 && !simple);
             if (cls == 1) {
                 const int nb = __popc(mk.x) + __popc(mk.y);
                 b_inter += nb;
@@ -565,45 +641,67 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 top += 2 * n_ow;
                 ptop += 2 * n_op;
             }
-            const int pcnt = __popc(m_pb);
+            // per-body items: the simple ones from the front of the list, the others (per-pair
+            // image or cut) from its end; lane l remembers the slot of its own
+            const int n_ps = __popc(m_ps), n_pg = __popc(m_pg);
+            int slot = -1;
             if (cls == 3) {
-                // the band [lo, hi] around s^2 / theta^2 inside which float64 decides
+                // the band [lo, hi] around s^2 / theta^2 inside which float64 decides.  A shifted
+                // CoM gives differences within 2^-25 + 2^-26 of the reference's, d^2 within
+                // 2 sqrt(3) d of that: 3e-7 d covers it twice.
                 const float R = s * s * inv_th2;
-                const int fl = (zero_image ? 0 : kItemWrap) | (near_box ? kItemNear : 0);
-                const int w = __popc(m_pb & lt);
-                plist[3 * w] = A;
-                plist[3 * w + 1] = make_float4(s, R * (1.f - kRelMargin), R * (1.f + kRelMargin),
-                                               __int_as_float(fl));
-                plist[3 * w + 2] = make_float4(__int_as_float(c0), __int_as_float(c1),
-                                               __uint_as_float(mk.x), __uint_as_float(mk.y));
+                const float widen = simple && shifted ? 3e-7f * sqrtf(R) : 0.f;
+                const float lo = R * (1.f - kRelMargin) - widen, hi = R * (1.f + kRelMargin) + widen;
+                const float m0 = __uint_as_float(mk.x), m1 = __uint_as_float(mk.y);
+                slot = simple ? __popc(m_ps & lt) : 31 - __popc(m_pg & lt);
+                float4 *item = plist + 3 * slot;
+                if (simple) {
+                    if (BPL == 2) {
+                        item[0] = make_float4(E.x, E.x, E.y, E.y);
+                        item[1] = make_float4(E.z, E.z, E.w, __int_as_float(node));
+                    } else {
+                        item[0] = E;
+                        item[1] = make_float4(0.f, 0.f, 0.f, __int_as_float(node));
+                    }
+                    item[2] = make_float4(lo, hi, m0, m1);
+                } else {
+                    const int fl = (one_image && !shifted ? 0 : kItemWrap) | (near_box ? kItemNear : 0);
+                    item[0] = A;
+                    item[1] = make_float4(s, lo, hi, __int_as_float(fl));
+                    item[2] = make_float4(0.f, 0.f, m0, m1);
+                }
             }
             __syncwarp();
-            // per-body items: every body of the mask decides for itself; lane j
-            // keeps item j's mask of opening bodies, and the children of every
-            // item that some body opened are pushed together afterwards
-            uint2 my_om = make_uint2(0u, 0u);
+            // every body of the mask decides for itself; a lane keeps the mask of the bodies that
+            // accept its own item, and the children of the items that some body opened are pushed
+            // together afterwards
+            uint2 my_acc = make_uint2(0u, 0u);
 #pragma unroll 1
-            for (int j = 0; j < pcnt; ++j) {
-                const float4 I = plist[3 * j], J = plist[3 * j + 1], K = plist[3 * j + 2];
+            for (int j = 0; j < n_ps; ++j) {
+                const uint2 acc = simple_item<BPL>(plist[3 * j], plist[3 * j + 1], plist[3 * j + 2],
+                                                   1u << lane, P.rec, P.box, th2d, soft2, x, y, z, ax,
+                                                   ay, az);
+                if (slot == j) my_acc = acc;
+            }
+#pragma unroll 1
+            for (int j = 31; j > 31 - n_pg; --j) {
+                const float4 K = plist[3 * j + 2];
                 bool opn[BPL];
-                per_body_item<BPL>(I, J, __float_as_uint(K.z), __float_as_uint(K.w), lane, th2d, soft2,
-                                   x, y, z, ax, ay, az, opn);
+                per_body_item<BPL>(plist[3 * j], plist[3 * j + 1], __float_as_uint(K.z),
+                                   __float_as_uint(K.w), lane, th2d, soft2, x, y, z, ax, ay, az, opn);
                 const uint32_t o0 = __ballot_sync(0xffffffffu, opn[0]);
                 const uint32_t o1 = BPL == 2 ? __ballot_sync(0xffffffffu, opn[BPL - 1]) : 0u;
-                if (lane == j) my_om = make_uint2(o0, o1);
+                if (slot == j) my_acc = make_uint2(~o0, ~o1);
             }
-            if (pcnt > 0) {
+            if (n_ps + n_pg > 0) {
+                uint2 my_om = make_uint2(0u, 0u);
                 bool has = false, whole_o = false;
-                int32_t k0 = -1, k1c = -1;
-                if (lane < pcnt) {
-                    const float4 K = plist[3 * lane + 2];
-                    k0 = __float_as_int(K.x);
-                    k1c = __float_as_int(K.y);
+                if (cls == 3) {
+                    my_om = make_uint2(mk.x & ~my_acc.x, mk.y & ~my_acc.y);
                     has = (my_om.x | my_om.y) != 0u;
                     whole_o = my_om.x == fm.x && my_om.y == fm.y;
                     // the bodies of the item's mask that did not open it accepted it
-                    n_acc += __popc(__float_as_uint(K.z)) + __popc(__float_as_uint(K.w)) -
-                             __popc(my_om.x) - __popc(my_om.y);
+                    n_acc += __popc(mk.x & my_acc.x) + __popc(mk.y & my_acc.y);
                 }
                 const uint32_t mw = __ballot_sync(0xffffffffu, has && whole_o);
                 const uint32_t mp = __ballot_sync(0xffffffffu, has && !whole_o);
@@ -614,16 +712,16 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 } else {
                     if (has && whole_o) {
                         const int pos = top + 2 * __popc(mw & lt);
-                        stack[pos] = k1c;
-                        stack[pos + 1] = k0;
+                        stack[pos] = c1;
+                        stack[pos + 1] = c0;
                     }
                     if (has && !whole_o) {
                         const int pos = ptop + 2 * __popc(mp & lt);
                         const int w1 = part_word<XW>(pos), w0 = part_word<XW>(pos + 1);
-                        stack[w1] = k1c;
+                        stack[w1] = c1;
                         stack[w1 + 1] = (int32_t)my_om.x;
                         stack[w1 + 2] = (int32_t)my_om.y;
-                        stack[w0] = k0;
+                        stack[w0] = c0;
                         stack[w0 + 1] = (int32_t)my_om.x;
                         stack[w0 + 2] = (int32_t)my_om.y;
                     }
