@@ -160,7 +160,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const float2 r = make_float2(rsqrtf(q[u].x), rsqrtf(q[u].y));
+                const float2 r = make_float2(rsqrt_normal(q[u].x), rsqrt_normal(q[u].y));
                 const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w[u], r), r), r);
                 fx = __ffma2_rn(f, dx[u], fx);
                 fy = __ffma2_rn(f, dy[u], fy);
@@ -183,7 +183,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
             const bool u0 = (mk.x & lane_bit) != 0u, u1 = (mk.y & lane_bit) != 0u;
             const float2 w = make_float2(u0 && (!WRAP_CUT || q.x > cut) ? b.z : 0.f,
                                          u1 && (!WRAP_CUT || q.y > cut) ? b.w : 0.f);
-            const float2 r = make_float2(rsqrtf(q.x), rsqrtf(q.y));
+            const float2 r = make_float2(rsqrt_normal(q.x), rsqrt_normal(q.y));
             const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, r), r), r);
             fx = __ffma2_rn(f, dx, fx);
             fy = __ffma2_rn(f, dy, fy);
@@ -206,7 +206,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
                     dz = minus_image(dz);
                 }
                 const float q = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
-                const float r = rsqrtf(q);
+                const float r = rsqrt_normal(q);
                 const float f = (u && (!WRAP_CUT || q > cut)) ? e.w * r * r * r : 0.f;
                 ax[b] = fmaf(f, dx, ax[b]);
                 ay[b] = fmaf(f, dy, ay[b]);
@@ -252,7 +252,7 @@ __device__ __forceinline__ void per_body_item(float4 I, float4 J, uint32_t m0, u
         // an item every reaching body opens adds no force (a third of them)
         if (!__any_sync(0xffffffffu, f0 || f1)) return;
         const float2 q = __fadd2_rn(d2, dup2(soft2));
-        const float2 r = make_float2(rsqrtf(q.x), rsqrtf(q.y));
+        const float2 r = make_float2(rsqrt_normal(q.x), rsqrt_normal(q.y));
         const float2 w = make_float2(f0 ? I.w : 0.f, f1 ? I.w : 0.f);
         const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, r), r), r);
         const float2 fx = __ffma2_rn(f, dx, make_float2(ax[0], ax[1]));
@@ -277,7 +277,7 @@ __device__ __forceinline__ void per_body_item(float4 I, float4 J, uint32_t m0, u
             const bool u = in && a;
             opn[b] = in && !a;
             const bool fu = u && (!(flags & kItemNear) || ref_outside_cut(dx, dy, dz, d2));
-            const float r = rsqrtf(d2 + soft2);
+            const float r = rsqrt_normal(d2 + soft2);
             const float f = fu ? I.w * r * r * r : 0.f;
             ax[b] = fmaf(f, dx, ax[b]);
             ay[b] = fmaf(f, dy, ay[b]);
@@ -326,7 +326,7 @@ __device__ __forceinline__ uint2 simple_item(float4 I, float4 J, float4 K, uint3
         // an item every reaching body opens adds no force (a third of them)
         if ((acc.x | acc.y) == 0u) return acc;
         const float2 q = __fadd2_rn(d2, dup2(soft2));
-        const float2 r = make_float2(rsqrtf(q.x), rsqrtf(q.y));
+        const float2 r = make_float2(rsqrt_normal(q.x), rsqrt_normal(q.y));
         const float2 w = make_float2(p0 ? J.z : 0.f, p1 ? J.z : 0.f);
         const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, r), r), r);
         const float2 fx = __ffma2_rn(f, dx, make_float2(ax[0], ax[1]));
@@ -344,7 +344,7 @@ __device__ __forceinline__ uint2 simple_item(float4 I, float4 J, float4 K, uint3
         p = p && (__float_as_uint(K.z) & lane_bit) != 0u;
         const uint32_t acc = __ballot_sync(0xffffffffu, p);
         if (acc == 0u) return make_uint2(0u, 0u);
-        const float r = rsqrtf(d2 + soft2);
+        const float r = rsqrt_normal(d2 + soft2);
         const float f = p ? I.w * r * r * r : 0.f;
         ax[0] = fmaf(f, dx, ax[0]);
         ay[0] = fmaf(f, dy, ay[0]);
@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
             soft2 = bp.y * bp.y;
             th2d = (double)th * (double)th;
         }
+        soft2 = fmaxf(soft2, kMinSoft2);
         if (P.theta_per_bucket) {
             th = P.theta_per_bucket[g];
             th2d = (double)th * (double)th;

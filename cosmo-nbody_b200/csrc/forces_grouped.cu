@@ -146,7 +146,7 @@ __device__ __forceinline__ void apply_quad(const float4 *q, int cnt, const float
             const float2 dx = __fadd2_rn(dup(e.x), nx), dy = __fadd2_rn(dup(e.y), ny),
                          dz = __fadd2_rn(dup(e.z), nz);
             const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, s2)));
-            const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+            const float2 ri = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
             const float2 ri2 = __fmul2_rn(ri, ri), ri3 = __fmul2_rn(ri2, ri);
             const float2 ri5 = __fmul2_rn(ri3, ri2), ri7 = __fmul2_rn(ri5, ri2);
             const float2 qx = __ffma2_rn(dup(u.x), dx, __ffma2_rn(dup(u.y), dy, __fmul2_rn(dup(u.z), dz)));
@@ -174,7 +174,7 @@ __device__ __forceinline__ void apply_quad(const float4 *q, int cnt, const float
         for (int b = 0; b < BPL; ++b) {
             const float dx = e.x - x[b], dy = e.y - y[b], dz = e.z - z[b];
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
-            const float ri = rsqrtf(r2);
+            const float ri = rsqrt_normal(r2);
             const float ri2 = ri * ri, ri3 = ri2 * ri, ri5 = ri3 * ri2, ri7 = ri5 * ri2;
             const float qx = fmaf(u.x, dx, fmaf(u.y, dy, u.z * dz));
             const float qy = fmaf(u.y, dx, fmaf(u.w, dy, v.x * dz));
@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
             soft2 = bp.y * bp.y;
             slab_mass = bp.z;
         }
+        soft2 = fmaxf(soft2, kMinSoft2);
         if (P.theta_per_bucket) th = P.theta_per_bucket[g];
         const float th2 = th * th;
 

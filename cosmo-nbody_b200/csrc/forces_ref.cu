@@ -11,6 +11,8 @@
 // reference (float32 node data, `round()` promoting the displacement);
 // T = float is the float32 form.  The reference's shared-memory copy of the
 // top 256 nodes only mirrors node data and is not needed for the result.
+#include <math.h>
+
 #include <type_traits>
 
 #include "grouped.cuh"
@@ -26,13 +28,13 @@ __device__ __forceinline__ T min_image(float d) {
     return (T)(d - rintf(d));
 }
 
-// q^(-3/2)
+// q^(-3/2); in float32 q is at least kMinSoft2
 __device__ __forceinline__ double inv_r3(double q) {
     const double r = rsqrt(q);
     return r * r * r;
 }
 __device__ __forceinline__ float inv_r3(float q) {
-    const float r = rsqrtf(q);
+    const float r = rsqrt_normal(q);
     return r * r * r;
 }
 
@@ -397,7 +399,7 @@ int launch_exact_walk(const GroupedParams &P, cudaStream_t st) {
     R.rec = P.rec;
     R.theta_sq = P.theta * P.theta;
     R.G = P.G;
-    R.soft2 = P.soft2;
+    R.soft2 = fmaxf(P.soft2, kMinSoft2);
     R.box = P.box;
     R.m_nodes = P.m_nodes;
     return forces_walk<float, true, true>(P.px, P.py, P.pz, R, P.theta_sq, P.force, nullptr, P.root, 0,
@@ -411,6 +413,7 @@ static int forces_ref(const float *px, const float *py, const float *pz, RefTree
     R.theta_sq = (T)(theta * theta);
     R.G = (T)G;
     R.soft2 = (T)(soft * soft);
+    if (sizeof(T) == 4) R.soft2 = R.soft2 > (T)kMinSoft2 ? R.soft2 : (T)kMinSoft2;
     R.box = (T)box;
     R.m_nodes = 2 * n - 1;
     if (count > n - off) count = n - off;
