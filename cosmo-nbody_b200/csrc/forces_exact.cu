@@ -29,11 +29,11 @@
 // reference.  The forces differ from the reference's only by float32 against
 // float64 arithmetic and summation order.
 //
-// Lists: entries with one image for every body of the bucket and out of the
-// cut's reach go to the whole-bucket list (applied as in forces_grouped.cu:
-// packed float2 for two bodies per lane, no image, no cut) or, reached by part
-// of the bucket, to the masked list (the same, the mass selected per body by
-// the entry's mask); every other accepted entry keeps the node's raw CoM and
+// Lists: entries with one image for every body of their mask and out of the
+// cut's reach go to the masked list (packed float2 for two bodies per lane, no
+// image, no cut, the mass selected per body by the entry's mask; whole-bucket
+// entries too: a list of their own saves them five instructions and costs
+// every round more); every other accepted entry keeps the node's raw CoM and
 // is applied with the per-pair minimum image, the cut and its mask.
 // Per-body items carry the band [lo, hi] around s^2 / theta^2 inside which
 // the float32 d^2 cannot decide.  Most are simple (87 % at 128^3): one image
@@ -59,24 +59,26 @@ namespace cnb {
 // The two node stacks of a warp share one region of XW words: entries
 // reached by the whole bucket (one word, the node) grow up from word 0,
 // entries reached by part of it (three words: node, mask low, mask high)
-// grow down from the end.  The main pass gives up on a bucket whose stacks
-// would meet (it marks the bucket's record and writes no force for it); a
-// second pass walks only those buckets again with a region of
-// kXWordsRedo words, and a push that would overflow that one drops the
-// children and flags CNB_FLAG_LIST_OVERFLOW.  The deepest use measured at
-// theta = 0.5 on 128^3 and 256^3 Zel'dovich and evolved states (two-level
-// walk included) is 568 words; 864 is the most that keeps ten 2-warp
-// blocks (20 warps) per SM; smaller angles walk deeper and start wider.
-constexpr int kXWords = 864;       // main pass, theta >= 0.4
-constexpr int kXWordsWide = 2048;  // main pass, theta < 0.4
+// grow down from the end.  A round pops no more entries than the free words
+// can take back, so a walk that fills the region narrows to a depth-first one
+// and only a path some thirty levels deeper still is given up by the main pass
+// (it marks the bucket's record and writes no force for it); a second pass
+// walks those buckets again with a region of kXWordsRedo words, and drops what
+// does not fit there (CNB_FLAG_LIST_OVERFLOW).  Rounds are full until 480 of
+// the 640 words are used; the deepest use at theta = 0.5 on 128^3 and 256^3
+// Zel'dovich and evolved states (two-level walk included) is 585 words.
+// 640 against 864 words (and 2048 at small angles or with several boxes, as
+// one size used to need): theta 0.3 500k bodies 4.72 -> 4.35 ms, 16 boxes
+// 1.48 -> 1.37; 512 and 496 are no faster.
+constexpr int kXWords = 640;       // main pass
 constexpr int kXWordsRedo = 4096;  // the buckets a main pass gave up on
 template <int XW> __device__ __forceinline__ int part_word(int k) { return XW - 3 * (k + 1); }
 
-// per-warp shared memory: the whole-bucket and masked lists (packed for two
-// bodies per lane), the per-pair list (one float4 per entry), the per-body
-// items of one round, the two lists' masks and the stack region
+// per-warp shared memory: the masked list (packed for two bodies per lane), the
+// per-pair list (one float4 per entry), the per-body items of one round, the
+// two lists' masks and the stack region
 template <int BPL> __host__ __device__ constexpr int exact_f4_per_warp() {
-    return 2 * kGList * entry_width<BPL>() + kGList + 3 * 32;
+    return kGList * entry_width<BPL>() + kGList + 3 * 32;
 }
 constexpr int kExactMasksPerWarp = 2 * kGList;  // uint2
 
@@ -138,10 +140,10 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
         // eight entries at a time: loads, distances and masses first, then the
         // inverse cubes and the accumulation in list order
         int j = 0;
-        for (; j + 8 <= cnt; j += 8) {
-            float2 dx[8], dy[8], dz[8], w[8], q[8];
+        for (; j + 4 <= cnt; j += 4) {
+            float2 dx[4], dy[4], dz[4], w[4], q[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < 4; ++u) {
                 float4 a, b;
                 entry_pair<WRAP_CUT>(list, j + u, a, b);
                 const uint2 mk = masks[j + u];
@@ -159,7 +161,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
                                    u1 && (!WRAP_CUT || q[u].y > cut) ? b.w : 0.f);
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < 4; ++u) {
                 const float2 r = make_float2(rsqrt_normal(q[u].x), rsqrt_normal(q[u].y));
                 const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(w[u], r), r), r);
                 fx = __ffma2_rn(f, dx[u], fx);
@@ -354,20 +356,19 @@ __device__ __forceinline__ uint2 simple_item(float4 I, float4 J, float4 K, uint3
 }
 
 // Applies the first 32 entries of a list and moves the rest to the front.
-template <int BPL, int KIND>
+// WRAP_CUT: the per-pair list (one float4 per entry), else the masked list.
+template <int BPL, bool WRAP_CUT>
 __device__ __forceinline__ void flush32(float4 *lst, uint2 *msk, int &cnt, int lane,
                                         const float (&x)[BPL], const float (&y)[BPL],
                                         const float (&z)[BPL], float soft2, float (&ax)[BPL],
                                         float (&ay)[BPL], float (&az)[BPL]) {
-    constexpr int EW = KIND == 2 ? 1 : entry_width<BPL>();  // the per-pair list: one float4
-    if (KIND == 0) apply_entries<BPL, false, false>(lst, 32, x, y, z, soft2, ax, ay, az);
-    else if (KIND == 1) apply_masked<BPL, false>(lst, msk, 32, lane, x, y, z, soft2, ax, ay, az);
-    else apply_masked<BPL, true>(lst, msk, 32, lane, x, y, z, soft2, ax, ay, az);
+    constexpr int EW = WRAP_CUT ? 1 : entry_width<BPL>();
+    apply_masked<BPL, WRAP_CUT>(lst, msk, 32, lane, x, y, z, soft2, ax, ay, az);
     __syncwarp();
 #pragma unroll
     for (int w = 0; w < EW; ++w)
         if (lane < cnt - 32) lst[EW * lane + w] = lst[EW * (32 + lane) + w];
-    if (KIND != 0 && lane < cnt - 32) msk[lane] = msk[32 + lane];
+    if (lane < cnt - 32) msk[lane] = msk[32 + lane];
     cnt -= 32;
     __syncwarp();
 }
@@ -375,18 +376,19 @@ __device__ __forceinline__ void flush32(float4 *lst, uint2 *msk, int &cnt, int l
 // REDO false: the main pass over every bucket (work counter); true: the
 // buckets a main pass gave up on (bucket record's fourth word = 1), found by
 // a strided scan of the table and cleared when done.
-// Twenty warps per SM: ten 2-warp blocks fit the shared memory of the main
-// pass; the register bound (at most 102 for 2 or 4 warps per block) keeps them.
+// Twenty warps per SM with two bodies per lane, 28 with one (24 in blocks of
+// eight).  Two bodies want their registers: bounded for 22 or 24 warps the
+// kernel is 2 % faster to 6 % slower at 2M bodies and 8 to 13 % slower at 300k.
+// One body leaves room: 128^3 one level 5.72 (16 warps) -> 4.88 ms (24).
 template <int BPL, int WARPS, int XW, bool REDO, bool TEST = false>
-__global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(GroupedParams P) {
+__global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_forces_exact(GroupedParams P) {
     static_assert(BPL == 1 || BPL == 2, "one or two bodies per lane");
     extern __shared__ __align__(16) unsigned char x_smem[];
     constexpr int EW = entry_width<BPL>();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     float4 *f4 = reinterpret_cast<float4 *>(x_smem);
-    float4 *list = f4 + wib * exact_f4_per_warp<BPL>();  // whole bucket, one image, no cut
-    float4 *mlist = list + kGList * EW;                   // masked, one image, no cut
+    float4 *mlist = f4 + wib * exact_f4_per_warp<BPL>();  // masked, one image, no cut
     float4 *xlist = mlist + kGList * EW;                  // per-pair image and cut, any mask
     float4 *plist = xlist + kGList;                       // per-body items (3 float4 each)
     uint2 *mbase = reinterpret_cast<uint2 *>(f4 + WARPS * exact_f4_per_warp<BPL>());
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
         float ax[BPL], ay[BPL], az[BPL];
 #pragma unroll
         for (int b = 0; b < BPL; ++b) ax[b] = ay[b] = az[b] = 0.f;
-        int top = 1, ptop = 0, cnt = 0, mcnt = 0, xcnt = 0, n_acc = 0;
+        int top = 1, ptop = 0, mcnt = 0, xcnt = 0, n_acc = 0;
         bool seeded = false;
         if (P.super_of_body) {
             const int sup = P.super_of_body[bk.x];
@@ -499,16 +501,16 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 const float4 *far = P.far_lists + (int64_t)sup * P.far_cap;
                 for (int j0 = 0; j0 < h.x; j0 += 32) {
                     const int c = min(32, h.x - j0);
-                    if (lane < c) put_entry<BPL>(list, lane, far[j0 + lane]);
+                    if (lane < c) put_entry<BPL>(mlist, lane, far[j0 + lane]);
                     __syncwarp();
-                    apply_entries<BPL, false, false>(list, c, x, y, z, soft2, ax, ay, az);
+                    apply_entries<BPL, false, false>(mlist, c, x, y, z, soft2, ax, ay, az);
                     __syncwarp();
                 }
                 for (int j0 = 0; j0 < h.y; j0 += 32) {
                     const int c = min(32, h.y - j0);
-                    if (lane < c) put_entry<BPL>(list, lane, far[P.far_cap - h.y + j0 + lane]);
+                    if (lane < c) put_entry<BPL>(mlist, lane, far[P.far_cap - h.y + j0 + lane]);
                     __syncwarp();
-                    apply_entries<BPL, true, true>(list, c, x, y, z, soft2, ax, ay, az);
+                    apply_entries<BPL, true, true>(mlist, c, x, y, z, soft2, ax, ay, az);
                     __syncwarp();
                 }
                 if (lane == 0) {
@@ -530,9 +532,18 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 if (lane == 0) set_flag(P.status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
+            // A popped entry leaves at most five words more than it took (a whole-bucket entry
+            // opened by part of the bucket: one word becomes two (node, mask) entries), so
+            // popping a fifth of the free words never overflows the region; a full one is spilt.
+            const int room = ((XW - top - 3 * ptop) * 51) >> 8;
+            if (room == 0) {
+                if (REDO) overflow = true;
+                spill = true;
+                break;
+            }
             // part-bucket entries first (they keep the second stack short)
-            const int k1 = ptop < 32 ? ptop : 32;
-            const int k2 = min(top, 32 - k1);
+            const int k1 = min(ptop, min(32, room));
+            const int k2 = min(top, min(32, room) - k1);
             ptop -= k1;
             top -= k2;
             int32_t node = -1;
@@ -549,7 +560,6 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 set_flag(P.status, CNB_FLAG_BAD_TOPOLOGY);
                 node = -1;
             }
-            const bool whole = mk.x == fm.x && mk.y == fm.y;
             // 1: accepted by every body of the mask, 2: opened by every one, 3: per body
             int cls = 0;
             bool one_image = false, simple = false, shifted = false, near_box = false;
@@ -590,22 +600,16 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 }
             }
             b_tests += (node >= 0);
-            const bool to_list = cls == 1 && whole && one_image && !near_box;
-            const bool to_m = cls == 1 && !whole && one_image && !near_box;
+            const bool to_m = cls == 1 && one_image && !near_box;
             const bool to_x = cls == 1 && !(one_image && !near_box);
-            const uint32_t m_one = __ballot_sync(0xffffffffu, to_list);
             const uint32_t m_msk = __ballot_sync(0xffffffffu, to_m);
             const uint32_t m_x = __ballot_sync(0xffffffffu, to_x);
-            const uint32_t m_ow = __ballot_sync(0xffffffffu, cls == 2 && whole);
-            const uint32_t m_op = __ballot_sync(0xffffffffu, cls == 2 && !whole);
             const uint32_t m_ps = __ballot_sync(0xffffffffu, cls == 3 && simple);
             const uint32_t m_pg = __ballot_sync(0xffffffffu, cls == 3 && !simple);
             if (cls == 1) {
                 const int nb = __popc(mk.x) + __popc(mk.y);
                 b_inter += nb;
-                if (to_list) {
-                    put_entry<BPL>(list, cnt + __popc(m_one & lt), E);
-                } else if (to_m) {
+                if (to_m) {
                     const int w = mcnt + __popc(m_msk & lt);
                     put_entry<BPL>(mlist, w, E);
                     mmask[w] = mk;
@@ -616,32 +620,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                     b_wrap += nb;
                 }
             }
-            cnt += __popc(m_one);
             mcnt += __popc(m_msk);
             xcnt += __popc(m_x);
-            const int n_ow = __popc(m_ow), n_op = __popc(m_op);
-            if (top + 2 * n_ow + 3 * (ptop + 2 * n_op) > XW) {
-                if (REDO) overflow = true;  // children dropped (flagged)
-                else spill = true;          // the redo pass walks this bucket again
-            } else {
-                if (cls == 2 && whole) {
-                    const int pos = top + 2 * __popc(m_ow & lt);
-                    stack[pos] = c1;
-                    stack[pos + 1] = c0;
-                }
-                if (cls == 2 && !whole) {
-                    const int pos = ptop + 2 * __popc(m_op & lt);
-                    const int w1 = part_word<XW>(pos), w0 = part_word<XW>(pos + 1);
-                    stack[w1] = c1;
-                    stack[w1 + 1] = (int32_t)mk.x;
-                    stack[w1 + 2] = (int32_t)mk.y;
-                    stack[w0] = c0;
-                    stack[w0 + 1] = (int32_t)mk.x;
-                    stack[w0 + 2] = (int32_t)mk.y;
-                }
-                top += 2 * n_ow;
-                ptop += 2 * n_op;
-            }
             // per-body items: the simple ones from the front of the list, the others (per-pair
             // image or cut) from its end; lane l remembers the slot of its own
             const int n_ps = __popc(m_ps), n_pg = __popc(m_pg);
@@ -682,7 +662,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                 const uint2 acc = simple_item<BPL>(plist[3 * j], plist[3 * j + 1], plist[3 * j + 2],
                                                    1u << lane, P.rec, P.box, th2d, soft2, x, y, z, ax,
                                                    ay, az);
-                if (slot == j) my_acc = acc;
+                if (lane == 0) *reinterpret_cast<uint2 *>(plist + 3 * j + 2) = acc;
             }
 #pragma unroll 1
             for (int j = 31; j > 31 - n_pg; --j) {
@@ -692,25 +672,24 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
                                    __float_as_uint(K.w), lane, th2d, soft2, x, y, z, ax, ay, az, opn);
                 const uint32_t o0 = __ballot_sync(0xffffffffu, opn[0]);
                 const uint32_t o1 = BPL == 2 ? __ballot_sync(0xffffffffu, opn[BPL - 1]) : 0u;
-                if (slot == j) my_acc = make_uint2(~o0, ~o1);
+                if (lane == 0) *reinterpret_cast<uint2 *>(plist + 3 * j + 2) = make_uint2(~o0, ~o1);
             }
-            if (n_ps + n_pg > 0) {
+            __syncwarp();
+            if (cls == 3) my_acc = *reinterpret_cast<uint2 *>(plist + 3 * slot + 2);
+            {
+                // the bodies of each node's mask that open it: all, or those that did not accept
                 uint2 my_om = make_uint2(0u, 0u);
-                bool has = false, whole_o = false;
+                if (cls == 2) my_om = mk;
                 if (cls == 3) {
                     my_om = make_uint2(mk.x & ~my_acc.x, mk.y & ~my_acc.y);
-                    has = (my_om.x | my_om.y) != 0u;
-                    whole_o = my_om.x == fm.x && my_om.y == fm.y;
-                    // the bodies of the item's mask that did not open it accepted it
                     n_acc += __popc(mk.x & my_acc.x) + __popc(mk.y & my_acc.y);
                 }
+                const bool has = (my_om.x | my_om.y) != 0u;
+                const bool whole_o = my_om.x == fm.x && my_om.y == fm.y;
                 const uint32_t mw = __ballot_sync(0xffffffffu, has && whole_o);
                 const uint32_t mp = __ballot_sync(0xffffffffu, has && !whole_o);
                 const int nw = __popc(mw), npart = __popc(mp);
-                if (top + 2 * nw + 3 * (ptop + 2 * npart) > XW) {
-                    if (REDO) overflow = true;  // children dropped (flagged)
-                    else spill = true;          // the redo pass walks this bucket again
-                } else {
+                {
                     if (has && whole_o) {
                         const int pos = top + 2 * __popc(mw & lt);
                         stack[pos] = c1;
@@ -732,9 +711,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
             }
             max_top = max(max_top, top + 3 * ptop);  // words of the stack region
             __syncwarp();
-            if (cnt >= 32) flush32<BPL, 0>(list, nullptr, cnt, lane, x, y, z, soft2, ax, ay, az);
-            if (mcnt >= 32) flush32<BPL, 1>(mlist, mmask, mcnt, lane, x, y, z, soft2, ax, ay, az);
-            if (xcnt >= 32) flush32<BPL, 2>(xlist, xmask, xcnt, lane, x, y, z, soft2, ax, ay, az);
+            if (mcnt >= 32) flush32<BPL, false>(mlist, mmask, mcnt, lane, x, y, z, soft2, ax, ay, az);
+            if (xcnt >= 32) flush32<BPL, true>(xlist, xmask, xcnt, lane, x, y, z, soft2, ax, ay, az);
             // tests: give up on a bucket after its first round as an overflow would
             if (TEST && rounds == 1 && g % P.test_spill_every == 0) spill = true;
         }
@@ -745,7 +723,6 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_forces_exact(Grouped
             __syncwarp();
             continue;
         }
-        apply_entries<BPL, false, false>(list, cnt, x, y, z, soft2, ax, ay, az);
         apply_masked<BPL, false>(mlist, mmask, mcnt, lane, x, y, z, soft2, ax, ay, az);
         apply_masked<BPL, true>(xlist, xmask, xcnt, lane, x, y, z, soft2, ax, ay, az);
         __syncwarp();
@@ -798,11 +775,8 @@ static int launch_exact_pass(GroupedParams &P, cudaStream_t st) {
 
 template <int BPL, int WARPS>
 static int launch_exact_shape(GroupedParams &P, cudaStream_t st) {
-    // the main pass: smaller angles walk deeper and start with the wide region
     if (P.test_spill_every > 0)  // tests: the main pass gives up on every n-th bucket
         CNB_TRY((launch_exact_pass<BPL, WARPS, kXWords, false, true>(P, st)));
-    else if (P.theta < 0.4f)
-        CNB_TRY((launch_exact_pass<BPL, WARPS, kXWordsWide, false>(P, st)));
     else
         CNB_TRY((launch_exact_pass<BPL, WARPS, kXWords, false>(P, st)));
     // the buckets it gave up on, if any (otherwise every warp scans its share of the
