@@ -535,8 +535,12 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
             // A popped entry leaves at most five words more than it took (a whole-bucket entry
             // opened by part of the bucket: one word becomes two (node, mask) entries), so
             // popping a fifth of the free words never overflows the region; a full one is spilt.
-            const int room = ((XW - top - 3 * ptop) * 51) >> 8;
-            if (room == 0) {
+            // The redo pass goes by the main pass's region for as long as that lasts: the same
+            // order of nodes, so the same sums.
+            const int used = top + 3 * ptop;
+            int room = ((kXWords - used) * 51) >> 8;
+            if (REDO && room <= 0) room = ((XW - used) * 51) >> 8;
+            if (room <= 0) {
                 if (REDO) overflow = true;
                 spill = true;
                 break;
