@@ -35,12 +35,17 @@
 //                     kernel): 3-D extent, or b_max with quadrupoles; every
 //                     accepted node at the image nearest the bucket centre for
 //                     the whole bucket, plus the periodic correction of every
-//                     accepted node, accumulated per lane while walking and
-//                     applied per body once per bucket (ewald.cu has the law).
-//                     With quadrupole moments the second list carries the
-//                     internal nodes with their second central moments (and
-//                     the first list keeps the cut); without, the entries near
-//                     the bucket's box (the cut's).
+//                     accepted node, accumulated per lane as the lists are
+//                     applied (a lane per entry: a round accepts only some of
+//                     its nodes) and applied per body once per bucket (ewald.cu
+//                     has the law).  With quadrupole moments the second list
+//                     carries the internal nodes with their second central
+//                     moments, and a list is applied with the cut while it holds
+//                     an entry near the bucket's box; without, the second list
+//                     holds those entries.  Looking the correction up while
+//                     walking and cutting every quadrupole pair: 128^3 4.41
+//                     against 4.31 ms, 30k bodies 182 against 143 us,
+//                     quadrupoles 300k theta 0.4 1.36 against 1.155 ms.
 // theta is one value or one per bucket (learned controller).
 //
 // Two bodies per lane run the force loop on packed float2 (FADD2 / FMUL2 /
@@ -51,16 +56,29 @@
 namespace cnb {
 
 
+// The point of the octant table nearest d (|d_i| <= 1/2), as i | j << 10 | k << 20:
+// found as a node is accepted and kept with its list entry, since the entry's
+// own coordinates give d back only to rounding, and the expansion about a
+// point's neighbour differs by its second-order terms.
+__device__ __forceinline__ uint32_t ewald_cell(int nt, float dx, float dy, float dz) {
+    const float sc = 2.f * nt;
+    const auto near = [&](float d) {  // nearest integer of |d| sc, from the sum's low bits
+        const float v = __fadd_rn(__fmul_rn(fabsf(d), sc), 8388608.f);
+        return min(__float_as_uint(v) & 0x3ffu, (uint32_t)nt);
+    };
+    return near(dx) | near(dy) << 10 | near(dz) << 20;
+}
+
 // Periodic correction of one accepted node, d = its CoM image minus the
-// bucket centre (|d_i| <= 1/2): g(d) and its Jacobian from the nearest
-// point of the octant table, g to first order about that point, signs from
-// g's symmetry (g_i odd in d_i, even in the other components).
-__device__ __forceinline__ void ewald_lookup(const float4 *__restrict__ T, int nt, float dx,
-                                             float dy, float dz, float (&g)[3], float (&J)[6]) {
+// bucket centre: g(d) and its Jacobian from the table point `cell`, g to
+// first order about that point, signs from g's symmetry (g_i odd in d_i, even
+// in the other components).
+__device__ __forceinline__ void ewald_lookup(const float4 *__restrict__ T, int nt, uint32_t cell,
+                                             float dx, float dy, float dz, float (&g)[3],
+                                             float (&J)[6]) {
     const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
     const float sc = 2.f * nt;
-    const int i = min(__float2int_rn(ax * sc), nt), j = min(__float2int_rn(ay * sc), nt),
-              k = min(__float2int_rn(az * sc), nt);
+    const int i = cell & 0x3ffu, j = (cell >> 10) & 0x3ffu, k = cell >> 20;
     const int64_t t = ((int64_t)i * (nt + 1) + j) * (nt + 1) + k;
     const float4 t0 = __ldg(T + 6 * t), t1 = __ldg(T + 6 * t + 1), t2 = __ldg(T + 6 * t + 2);
     const float h = 1.f / sc;
@@ -82,13 +100,12 @@ __device__ __forceinline__ void ewald_lookup(const float4 *__restrict__ T, int n
 }
 
 // The periodic part of a node's quadrupole force, (1/2) H(d) : M2, with H
-// (the second derivatives of g) at the table point nearest d and M2 the
+// (the second derivatives of g) at the table point `cell` and M2 the
 // node's second central moment (xx, xy, xz, yy | yz, zz).
-__device__ __forceinline__ void ewald_quad(const float4 *__restrict__ T, int nt, float dx, float dy,
-                                           float dz, float4 ma, float4 mb, float (&out)[3]) {
-    const float sc = 2.f * nt;
-    const int i = min(__float2int_rn(fabsf(dx) * sc), nt), j = min(__float2int_rn(fabsf(dy) * sc), nt),
-              k = min(__float2int_rn(fabsf(dz) * sc), nt);
+__device__ __forceinline__ void ewald_quad(const float4 *__restrict__ T, int nt, uint32_t cell,
+                                           float dx, float dy, float dz, float4 ma, float4 mb,
+                                           float (&out)[3]) {
+    const int i = cell & 0x3ffu, j = (cell >> 10) & 0x3ffu, k = cell >> 20;
     const int64_t t = ((int64_t)i * (nt + 1) + j) * (nt + 1) + k;
     const float4 h0 = __ldg(T + 6 * t + 3), h1 = __ldg(T + 6 * t + 4), h2 = __ldg(T + 6 * t + 5);
     const float sx = dx < 0.f ? -1.f : 1.f, sy = dy < 0.f ? -1.f : 1.f, sz = dz < 0.f ? -1.f : 1.f;
@@ -104,11 +121,11 @@ __device__ __forceinline__ void ewald_quad(const float4 *__restrict__ T, int nt,
 }
 
 
-// float4 slots per entry of the second list: the per-pair-image list, or
-// under the periodic law the quadrupole list (position and mass | xx, xy, xz,
-// yy | yz, zz, trace, 0 of the node's second central moment)
-template <int BPL, bool EWALD> __host__ __device__ constexpr int second_width() {
-    return EWALD ? 3 : entry_width<BPL>();
+// float4 slots per entry of the second list: the monopole layout, or with
+// quadrupoles (position and mass | -3 (xx, xy, xz, yy) | -3 (yz, zz), -3/2
+// trace, 0 of the node's second central moment)
+template <int BPL, bool QUAD> __host__ __device__ constexpr int second_width() {
+    return QUAD ? 3 : entry_width<BPL>();
 }
 
 // The exact minimum-image test (CNB_MAC_PERIODIC) opens every node whose
@@ -116,17 +133,25 @@ template <int BPL, bool EWALD> __host__ __device__ constexpr int second_width() 
 // its node stack is this many entries per warp.
 constexpr int kGStackPeriodic = 4096;
 
-template <int BPL, bool EWALD>
+// the table points of the two lists' entries (quadrupole entries hold their own)
+template <int LAW> __host__ __device__ constexpr int cell_words() {
+    return LAW == 0 ? 0 : LAW == 1 ? 2 * kGList : kGList;
+}
+
+template <int BPL, int LAW>
 constexpr size_t grouped_smem(int warps, int stack) {
-    return (size_t)warps * (stack * sizeof(int32_t) +
-                            kGList * (entry_width<BPL>() + second_width<BPL, EWALD>()) *
+    constexpr bool QUAD = LAW == 2;
+    return (size_t)warps * ((stack + cell_words<LAW>()) * sizeof(int32_t) +
+                            kGList * (entry_width<BPL>() + second_width<BPL, QUAD>()) *
                                 sizeof(float4));
 }
 
 // Applies cnt quadrupole entries: per body the softened monopole plus
 // (15/2)(d.M d) d / r^7 - 3 M d / r^5 - (3/2) tr(M) d / r^5 for the node's
-// second central moment M about its CoM (d = CoM - body, r softened).
-template <int BPL>
+// second central moment M about its CoM (d = CoM - body, r softened), as
+// (m + (t - (5/2) d.q / r^2) / r^2) d / r^3 + q / r^5 with q = (-3 M) d and
+// t = -(3/2) tr(M), both as the entries hold them.  CUT: the reference's cut.
+template <int BPL, bool CUT>
 __device__ __forceinline__ void apply_quad(const float4 *q, int cnt, const float (&x)[BPL],
                                            const float (&y)[BPL], const float (&z)[BPL],
                                            float soft2, float (&ax)[BPL], float (&ay)[BPL],
@@ -146,21 +171,21 @@ __device__ __forceinline__ void apply_quad(const float4 *q, int cnt, const float
             const float2 dx = __fadd2_rn(dup(e.x), nx), dy = __fadd2_rn(dup(e.y), ny),
                          dz = __fadd2_rn(dup(e.z), nz);
             const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, s2)));
-            const float2 ri = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
-            const float2 ri2 = __fmul2_rn(ri, ri), ri3 = __fmul2_rn(ri2, ri);
-            const float2 ri5 = __fmul2_rn(ri3, ri2), ri7 = __fmul2_rn(ri5, ri2);
+            float2 ri = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
+            if (CUT) {
+                ri.x = r2.x > cut ? ri.x : 0.f;
+                ri.y = r2.y > cut ? ri.y : 0.f;
+            }
+            const float2 ri2 = __fmul2_rn(ri, ri), ri3 = __fmul2_rn(ri2, ri), ri5 = __fmul2_rn(ri3, ri2);
             const float2 qx = __ffma2_rn(dup(u.x), dx, __ffma2_rn(dup(u.y), dy, __fmul2_rn(dup(u.z), dz)));
             const float2 qy = __ffma2_rn(dup(u.y), dx, __ffma2_rn(dup(u.w), dy, __fmul2_rn(dup(v.x), dz)));
             const float2 qz = __ffma2_rn(dup(u.z), dx, __ffma2_rn(dup(v.x), dy, __fmul2_rn(dup(v.y), dz)));
             const float2 sq = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
-            float2 A = __ffma2_rn(dup(e.w), ri3,
-                                  __ffma2_rn(__fmul2_rn(dup(7.5f), sq), ri7, __fmul2_rn(dup(-1.5f * v.z), ri5)));
-            float2 B = __fmul2_rn(dup(-3.f), ri5);
-            if (!(r2.x > cut)) A.x = B.x = 0.f;
-            if (!(r2.y > cut)) A.y = B.y = 0.f;
-            fx = __ffma2_rn(A, dx, __ffma2_rn(B, qx, fx));
-            fy = __ffma2_rn(A, dy, __ffma2_rn(B, qy, fy));
-            fz = __ffma2_rn(A, dz, __ffma2_rn(B, qz, fz));
+            const float2 t = __ffma2_rn(sq, __fmul2_rn(dup(-2.5f), ri2), dup(v.z));
+            const float2 A = __fmul2_rn(ri3, __ffma2_rn(t, ri2, dup(e.w)));
+            fx = __ffma2_rn(A, dx, __ffma2_rn(ri5, qx, fx));
+            fy = __ffma2_rn(A, dy, __ffma2_rn(ri5, qy, fy));
+            fz = __ffma2_rn(A, dz, __ffma2_rn(ri5, qz, fz));
         }
         ax[0] = fx.x; ax[1] = fx.y;
         ay[0] = fy.x; ay[1] = fy.y;
@@ -174,26 +199,53 @@ __device__ __forceinline__ void apply_quad(const float4 *q, int cnt, const float
         for (int b = 0; b < BPL; ++b) {
             const float dx = e.x - x[b], dy = e.y - y[b], dz = e.z - z[b];
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
-            const float ri = rsqrt_normal(r2);
-            const float ri2 = ri * ri, ri3 = ri2 * ri, ri5 = ri3 * ri2, ri7 = ri5 * ri2;
+            float ri = rsqrt_normal(r2);
+            if (CUT) ri = r2 > cut ? ri : 0.f;
+            const float ri2 = ri * ri, ri3 = ri2 * ri, ri5 = ri3 * ri2;
             const float qx = fmaf(u.x, dx, fmaf(u.y, dy, u.z * dz));
             const float qy = fmaf(u.y, dx, fmaf(u.w, dy, v.x * dz));
             const float qz = fmaf(u.z, dx, fmaf(v.x, dy, v.y * dz));
             const float sq = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
-            float A = fmaf(e.w, ri3, fmaf(7.5f * sq, ri7, -1.5f * v.z * ri5));
-            float B = -3.f * ri5;
-            if (!(r2 > cut)) A = B = 0.f;
-            ax[b] = fmaf(A, dx, fmaf(B, qx, ax[b]));
-            ay[b] = fmaf(A, dy, fmaf(B, qy, ay[b]));
-            az[b] = fmaf(A, dz, fmaf(B, qz, az[b]));
+            const float A = ri3 * fmaf(fmaf(sq, -2.5f * ri2, v.z), ri2, e.w);
+            ax[b] = fmaf(A, dx, fmaf(ri5, qx, ax[b]));
+            ay[b] = fmaf(A, dy, fmaf(ri5, qy, ay[b]));
+            az[b] = fmaf(A, dz, fmaf(ri5, qz, az[b]));
         }
     }
 }
 
+// EWALD: the periodic correction of one applied entry (its image at d from
+// the bucket centre, mass m), added to a lane's sums m (c - centre), m, m g, m J.
+struct EwaldSums {
+    float c[4], g[3], j[6];
+    __device__ __forceinline__ void add(const float4 *T, int nt, uint32_t cell, float dx, float dy,
+                                        float dz, float m) {
+        float g_[3], J_[6];
+        ewald_lookup(T, nt, cell, dx, dy, dz, g_, J_);
+        c[0] = fmaf(m, dx, c[0]);
+        c[1] = fmaf(m, dy, c[1]);
+        c[2] = fmaf(m, dz, c[2]);
+        c[3] += m;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) g[q] = fmaf(m, g_[q], g[q]);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) j[q] = fmaf(m, J_[q], j[q]);
+    }
+};
+
 // LAW: 0 the minimum-image laws (CNB_MAC_REF_X, CNB_MAC_PERIODIC), 1 the
 // periodic (Ewald) law with monopoles, 2 the periodic law with quadrupoles.
+// Warps per SM the registers are bounded for, by measurement: law 0 24 (77 registers: 128^3 bucket
+// test 2.00 ms; 28 and 20: 2.02, 2.06), with the large stack 8 (128 registers: shared memory
+// keeps it at 11 warps anyway, 30k bodies 1.31 ms against 1.42 with 66 registers); law 1 28 (72
+// registers: 128^3 4.31 ms; left alone the compiler takes 64 and 4.48 ms), law 2 20 (95 registers:
+// 300k bodies 1.155 ms; 24: 1.23).
+template <int LAW, int STACK> __host__ __device__ constexpr int law_warps() {
+    return LAW == 1 ? 28 : LAW == 2 ? 20 : STACK > kGStack ? 8 : 24;
+}
+
 template <int BPL, int WARPS, int LAW, int STACK>
-__global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) {
+__global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k_forces_grouped(GroupedParams P) {
     constexpr bool EWALD = LAW != 0;
     constexpr bool QUAD = LAW == 2;
     extern __shared__ __align__(16) unsigned char g_smem[];
@@ -203,12 +255,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
     // bucket, and entries needing the per-pair image (under the periodic law:
     // internal nodes with their quadrupole moments)
     constexpr int EW = entry_width<BPL>();
-    constexpr int SW = second_width<BPL, EWALD>();
+    constexpr int SW = second_width<BPL, QUAD>();
     float4 *list = reinterpret_cast<float4 *>(g_smem) + wib * kGList * (EW + SW);
     float4 *wlist = list + kGList * EW;
     int32_t *stack =
         reinterpret_cast<int32_t *>(g_smem + WARPS * kGList * (EW + SW) * sizeof(float4)) +
-        wib * STACK;
+        wib * (STACK + cell_words<LAW>());
+    uint32_t *cells = reinterpret_cast<uint32_t *>(stack + STACK);
     unsigned long long n_tests = 0;
     int max_top = 0;
     bool overflow = false;
@@ -272,11 +325,11 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
         float ax[BPL], ay[BPL], az[BPL];
 #pragma unroll
         for (int b = 0; b < BPL; ++b) ax[b] = ay[b] = az[b] = 0.f;
-        // EWALD: this lane's share of sum m (c - centre), sum m, sum m g, sum m J
-        float ec[4] = {0.f, 0.f, 0.f, 0.f}, eg[3] = {0.f, 0.f, 0.f};
-        float ej[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        EwaldSums es{};  // EWALD: this lane's share
         int top = 1, cnt = 0, wcnt = 0;
-        unsigned long long n_entries = 0, n_wrap = 0;
+        uint32_t n_entries = 0, n_wrap = 0;
+        // QUAD: the first / second list holds an entry the cut can reach
+        bool cut1 = false, cut2 = false;
         bool seeded = false;
         if (P.super_of_body) {
             const int sup = P.super_of_body[bk.x];
@@ -309,6 +362,55 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
         }
         if (!seeded && lane == 0) stack[0] = root;
         __syncwarp();
+        // applies the first c entries of the first / the second list
+        const auto flush1 = [&](int c) {
+            if (EWALD && lane < c) {
+                const float4 h = list[EW * lane];
+                float4 e = h;
+                if (BPL == 2) {
+                    const float4 h1 = list[EW * lane + EW - 1];
+                    e = make_float4(h.x, h.z, h1.x, h1.z);
+                }
+                es.add(P.ewald, P.ewald_nt, cells[lane], e.x - gcx, e.y - gcy, e.z - gcz, e.w);
+            }
+            if (QUAD && cut1)
+                apply_entries<BPL, false, true>(list, c, x, y, z, soft2, ax, ay, az);
+            else
+                apply_entries<BPL, false, false>(list, c, x, y, z, soft2, ax, ay, az);
+            n_entries += c;
+        };
+        const auto flush2 = [&](int c) {
+            if (EWALD && lane < c) {
+                const int ww = QUAD ? SW : EW;
+                const float4 h = wlist[ww * lane];
+                float4 e = h;
+                if (!QUAD && BPL == 2) {
+                    const float4 h1 = wlist[ww * lane + 1];
+                    e = make_float4(h.x, h.z, h1.x, h1.z);
+                }
+                const uint32_t cl = QUAD ? __float_as_uint(wlist[ww * lane + 2].w) : cells[kGList + lane];
+                const float dx = e.x - gcx, dy = e.y - gcy, dz = e.z - gcz;
+                es.add(P.ewald, P.ewald_nt, cl, dx, dy, dz, e.w);
+                if (QUAD) {
+                    // and the periodic part of its quadrupole, a bucket constant
+                    float pq[3];
+                    ewald_quad(P.ewald, P.ewald_nt, cl, dx, dy, dz, wlist[3 * lane + 1],
+                               wlist[3 * lane + 2], pq);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) es.g[q] = fmaf(pq[q], -1.f / 3.f, es.g[q]);
+                }
+            }
+            if (QUAD && cut2)
+                apply_quad<BPL, true>(wlist, c, x, y, z, soft2, ax, ay, az);
+            else if (QUAD)
+                apply_quad<BPL, false>(wlist, c, x, y, z, soft2, ax, ay, az);
+            else if (EWALD)
+                apply_entries<BPL, false, true>(wlist, c, x, y, z, soft2, ax, ay, az);
+            else
+                apply_entries<BPL, true, true>(wlist, c, x, y, z, soft2, ax, ay, az);
+            n_entries += c;
+            n_wrap += c;
+        };
         // a valid tree pushes every node at most once per bucket: more rounds
         // than nodes means a cyclic topology
         int64_t rounds = 0;
@@ -328,6 +430,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
             }
             bool accept = false, open = false, consistent = true, near_box = false;
             float4 E = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t cell = 0;  // EWALD: the node's table point
             int32_t c0 = -1, c1 = -1;
             if (node >= 0) {
                 // both halves of the record (one 32-byte sector) in flight together
@@ -375,18 +478,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
                         const bool same_image = EWALD || (consistent &&
                             fabsf(dx) < wlx && fabsf(dy) < wly && fabsf(dz) < wlz);
                         E = make_float4(A.x - sx_, A.y - sy_, A.z - sz_, same_image ? A.w : -A.w);
-                        if (EWALD) {
-                            float g[3], J[6];
-                            ewald_lookup(P.ewald, P.ewald_nt, dx, dy, dz, g, J);
-                            ec[0] = fmaf(A.w, dx, ec[0]);
-                            ec[1] = fmaf(A.w, dy, ec[1]);
-                            ec[2] = fmaf(A.w, dz, ec[2]);
-                            ec[3] += A.w;
-#pragma unroll
-                            for (int q = 0; q < 3; ++q) eg[q] = fmaf(A.w, g[q], eg[q]);
-#pragma unroll
-                            for (int q = 0; q < 6; ++q) ej[q] = fmaf(A.w, J[q], ej[q]);
-                        }
+                        if (EWALD) cell = ewald_cell(P.ewald_nt, dx, dy, dz);
                     }
                 }
             }
@@ -394,33 +486,36 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
             const uint32_t am = __ballot_sync(0xffffffffu, accept);
             const uint32_t om = __ballot_sync(0xffffffffu, open);
             // second list: per-pair image, or (periodic law) an internal node's quadrupole;
-            // also every entry near enough to the box for the cut to apply, except with
-            // quadrupoles (the first list then keeps the cut)
+            // also every entry near enough to the box for the cut to apply (with quadrupoles
+            // those stay in their list, which is then applied with the cut)
             const bool to_w = EWALD ? (accept && (QUAD ? c0 != -1 : near_box))
                                     : (accept && (E.w < 0.f || near_box));
             const uint32_t wm = __ballot_sync(0xffffffffu, to_w);
             const uint32_t nm = am & ~wm;
+            if (QUAD) {
+                cut1 |= __any_sync(0xffffffffu, accept && near_box && !to_w) != 0;
+                cut2 |= __any_sync(0xffffffffu, to_w && near_box) != 0;
+            }
             if (accept) {
                 if (to_w) {
                     const int w = wcnt + __popc(wm & lt);
                     if (EWALD && !QUAD) {
                         put_entry<BPL>(wlist, w, E);  // near the box: a monopole with the cut
+                        cells[kGList + w] = cell;
                     } else if (EWALD) {
                         const float4 qa = __ldg(P.quad + 2 * node), qb = __ldg(P.quad + 2 * node + 1);
                         wlist[3 * w] = E;
-                        wlist[3 * w + 1] = qa;
-                        wlist[3 * w + 2] = make_float4(qb.x, qb.y, qa.x + qa.w + qb.y, 0.f);
-                        // and the periodic part of its quadrupole, a bucket constant
-                        float pq[3];
-                        ewald_quad(P.ewald, P.ewald_nt, E.x - gcx, E.y - gcy, E.z - gcz, qa, qb, pq);
-                        eg[0] += pq[0];
-                        eg[1] += pq[1];
-                        eg[2] += pq[2];
+                        wlist[3 * w + 1] = make_float4(-3.f * qa.x, -3.f * qa.y, -3.f * qa.z, -3.f * qa.w);
+                        wlist[3 * w + 2] = make_float4(-3.f * qb.x, -3.f * qb.y,
+                                                       -1.5f * (qa.x + qa.w + qb.y),
+                                                       __uint_as_float(cell));
                     } else {
                         put_entry<BPL>(wlist, w, make_float4(E.x, E.y, E.z, fabsf(E.w)));
                     }
                 } else {
-                    put_entry<BPL>(list, cnt + __popc(nm & lt), E);
+                    const int w = cnt + __popc(nm & lt);
+                    put_entry<BPL>(list, w, E);
+                    if (EWALD) cells[w] = cell;
                 }
             }
             cnt += __popc(nm);
@@ -439,49 +534,32 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
             }
             __syncwarp();
             if (cnt >= 32) {
-                if (QUAD)
-                    apply_entries<BPL, false, true>(list, 32, x, y, z, soft2, ax, ay, az);
-                else
-                    apply_entries<BPL, false, false>(list, 32, x, y, z, soft2, ax, ay, az);
-                n_entries += 32;
+                flush1(32);
                 __syncwarp();
 #pragma unroll
                 for (int w = 0; w < EW; ++w)
                     if (lane < cnt - 32) list[EW * lane + w] = list[EW * (32 + lane) + w];
+                if (EWALD && lane < cnt - 32) cells[lane] = cells[32 + lane];
                 cnt -= 32;
+                if (cnt == 0) cut1 = false;
                 __syncwarp();
             }
             if (wcnt >= 32) {
-                if (QUAD)
-                    apply_quad<BPL>(wlist, 32, x, y, z, soft2, ax, ay, az);
-                else if (EWALD)
-                    apply_entries<BPL, false, true>(wlist, 32, x, y, z, soft2, ax, ay, az);
-                else
-                    apply_entries<BPL, true, true>(wlist, 32, x, y, z, soft2, ax, ay, az);
-                n_entries += 32;
-                n_wrap += 32;
+                flush2(32);
                 __syncwarp();
-                // float4 slots per entry: quadrupole entries, or the monopole layout
-                const int ww = (QUAD) ? SW : EW;
+                const int ww = QUAD ? SW : EW;  // float4 slots per entry
 #pragma unroll
                 for (int w = 0; w < SW; ++w)
                     if (w < ww && lane < wcnt - 32) wlist[ww * lane + w] = wlist[ww * (32 + lane) + w];
+                if (EWALD && !QUAD && lane < wcnt - 32)
+                    cells[kGList + lane] = cells[kGList + 32 + lane];
                 wcnt -= 32;
+                if (wcnt == 0) cut2 = false;
                 __syncwarp();
             }
         }
-        if (QUAD)
-            apply_entries<BPL, false, true>(list, cnt, x, y, z, soft2, ax, ay, az);
-        else
-            apply_entries<BPL, false, false>(list, cnt, x, y, z, soft2, ax, ay, az);
-        if (QUAD)
-            apply_quad<BPL>(wlist, wcnt, x, y, z, soft2, ax, ay, az);
-        else if (EWALD)
-            apply_entries<BPL, false, true>(wlist, wcnt, x, y, z, soft2, ax, ay, az);
-        else
-            apply_entries<BPL, true, true>(wlist, wcnt, x, y, z, soft2, ax, ay, az);
-        n_entries += cnt + wcnt;
-        n_wrap += wcnt;
+        flush1(cnt);
+        flush2(wcnt);
         __syncwarp();
         if (EWALD) {
             // bucket totals, then per body the periodic correction of every
@@ -490,22 +568,22 @@ __global__ void __launch_bounds__(WARPS * 32) k_forces_grouped(GroupedParams P) 
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) ec[q] += __shfl_xor_sync(0xffffffffu, ec[q], o);
+                for (int q = 0; q < 4; ++q) es.c[q] += __shfl_xor_sync(0xffffffffu, es.c[q], o);
 #pragma unroll
-                for (int q = 0; q < 3; ++q) eg[q] += __shfl_xor_sync(0xffffffffu, eg[q], o);
+                for (int q = 0; q < 3; ++q) es.g[q] += __shfl_xor_sync(0xffffffffu, es.g[q], o);
 #pragma unroll
-                for (int q = 0; q < 6; ++q) ej[q] += __shfl_xor_sync(0xffffffffu, ej[q], o);
+                for (int q = 0; q < 6; ++q) es.j[q] += __shfl_xor_sync(0xffffffffu, es.j[q], o);
             }
             const float lin = 4.18879020478639f;  // 4 pi / 3
 #pragma unroll
             for (int b = 0; b < BPL; ++b) {
                 const float ux = gcx - x[b], uy = gcy - y[b], uz = gcz - z[b];
                 // sum m (c - x) = sum m (c - centre) + M (centre - x)
-                const float cx = fmaf(ec[3], ux, ec[0]), cy = fmaf(ec[3], uy, ec[1]),
-                            cz = fmaf(ec[3], uz, ec[2]);
-                ax[b] += eg[0] + ej[0] * ux + ej[1] * uy + ej[2] * uz - lin * cx;
-                ay[b] += eg[1] + ej[1] * ux + ej[3] * uy + ej[4] * uz - lin * cy;
-                az[b] += eg[2] + ej[2] * ux + ej[4] * uy + ej[5] * uz - lin * cz;
+                const float cx = fmaf(es.c[3], ux, es.c[0]), cy = fmaf(es.c[3], uy, es.c[1]),
+                            cz = fmaf(es.c[3], uz, es.c[2]);
+                ax[b] += es.g[0] + es.j[0] * ux + es.j[1] * uy + es.j[2] * uz - lin * cx;
+                ay[b] += es.g[1] + es.j[1] * ux + es.j[3] * uy + es.j[4] * uz - lin * cy;
+                az[b] += es.g[2] + es.j[2] * ux + es.j[4] * uy + es.j[5] * uz - lin * cz;
             }
         }
 #pragma unroll
@@ -786,7 +864,7 @@ extern "C" int cnb_pack_nodes(const float *n_mass, const float *n_com, const flo
 
 template <int BPL, int WARPS, int LAW, int STACK>
 static int launch_shape(GroupedParams &P, cudaStream_t st) {
-    const size_t smem = grouped_smem<BPL, LAW != 0>(WARPS, STACK);
+    const size_t smem = grouped_smem<BPL, LAW>(WARPS, STACK);
     CNB_CUDA(cudaFuncSetAttribute(k_forces_grouped<BPL, WARPS, LAW, STACK>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
