@@ -24,6 +24,7 @@ struct cnb_ctx {
     int32_t wait_limit = 0;          // look-back polls before a wait gives up (0: 2^22)
     int64_t withheld_tile = -1;      // one-sweep tile that never publishes its counts
     int64_t near_dest_bias = 0;      // added to the near-sorted path's R destinations
+    int persistent_blocks = 0;       // resident blocks of the persistent sort (0: not available)
     // grouped traversal scratch (grown on demand by cnb_forces_grouped)
     void *group_scratch = nullptr;
     size_t group_scratch_bytes = 0;
@@ -38,10 +39,19 @@ constexpr int kNearCap = 2048;                        // at most this many keys 
 int64_t near_bytes(int64_t n_max);
 int sort_pairs_near(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
                     uint32_t *perm_out, int64_t n, cudaStream_t st, const int32_t **skip_full,
-                    const int32_t **never, cudaGraphConditionalHandle cond, bool use_cond);
+                    const int32_t **never, uint32_t **arrivals, cudaGraphConditionalHandle cond,
+                    bool use_cond);
 int sort_pairs_onesweep(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
                         const uint32_t *idx_in, uint32_t *perm_out, int64_t n, int key_bits,
                         cudaStream_t st, const int32_t *skip = nullptr);
+
+// The full sort as one cooperative launch (sort_persistent.cu).  arrivals: a
+// zeroed word for its barriers, or null (it zeroes one itself).
+int persistent_blocks();
+int64_t persistent_max(const cnb_ctx *ctx);
+int sort_pairs_persistent(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
+                          const uint32_t *idx_in, uint32_t *perm_out, int64_t n, int key_bits,
+                          cudaStream_t st, const int32_t *skip, uint32_t *arrivals);
 
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;

@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     }
     __syncwarp();
     while (top > 0) {
-        const int k = top < 32 ? top : 32;
+        // fewer as the stack fills (a popped entry leaves at most one more than it took), so that
+        // a walk that opens everything narrows to a depth-first one
+        const int room = (kRefStack - top) >> 3;
+        const int k = min(top, min(32, room > 1 ? room : 1));
         top -= k;
         popped += k;
         int2 ch = make_int2(-1, -1);

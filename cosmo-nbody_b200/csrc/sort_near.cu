@@ -59,7 +59,8 @@ static_assert(kNearWin < 65536, "window positions are 16-bit");
 static_assert(kNearItems == 8 && kNearTile % 32 == 0, "eight keys per thread, one byte of a word");
 
 struct NearWs {
-    int32_t *ctl;  // [0] give up, [1] near path taken, [2] |S|, [3..5] blocks done per kernel
+    int32_t *ctl;  // [0] give up, [1] near path taken, [2] |S|, [3..5] blocks done per kernel,
+                   // [6] the persistent full sort's barrier arrivals
     uint64_t *umax, *umin, *pmax, *smin, *rkey;  // per tile
     uint32_t *scnt, *soff, *rpos, *dirty, *tlo;  // per tile (soff, tlo: tiles + 1)
     uint32_t *bits;                              // per tile kNearWords words
@@ -656,12 +657,13 @@ int64_t near_bytes(int64_t n_max) {
 
 // Launches the near-sorted path; *skip_full receives the device flag that
 // is non-zero when it produced the result (the full sort's kernels then
-// return), *never a device flag that stays zero.  use_cond: the launches are
+// return), *never a device flag that stays zero, *arrivals a zeroed word.  use_cond: the launches are
 // being captured into a CUDA graph whose conditional node `cond` holds the
 // full sort; the path sets it to 0 when it produced the result.
 int sort_pairs_near(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
                     uint32_t *perm_out, int64_t n, cudaStream_t st, const int32_t **skip_full,
-                    const int32_t **never, cudaGraphConditionalHandle cond, bool use_cond) {
+                    const int32_t **never, uint32_t **arrivals, cudaGraphConditionalHandle cond,
+                    bool use_cond) {
     const int64_t nt = (n + kNearTile - 1) / kNearTile;
     const int64_t nt_max = (ctx->n_max + kNearTile - 1) / kNearTile;
     NearWs w;
@@ -684,6 +686,7 @@ int sort_pairs_near(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
     CNB_TRY(launch_status());
     *skip_full = w.ctl + 1;
     *never = w.ctl + 7;  // zeroed with the rest of ctl, never set
+    *arrivals = reinterpret_cast<uint32_t *>(w.ctl + 6);  // zeroed too
     return CNB_OK;
 }
 

@@ -170,3 +170,29 @@ def test_redo_pass_past_the_rule(theta):
         assert int(status.item()) == 0
         out.append(f.cpu().numpy().view(np.uint32))
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n,spread", [(30000, 0.2), (30000, 1e-3)])
+def test_walk_that_opens_everything(n, spread):
+    """theta = 0: every body meets every body, through a stack that would
+    overflow if every round took 32 nodes."""
+    from cnb import _lib
+    from cnb.core.octree import OctreeManager
+    rng = np.random.default_rng(n)
+    p = (0.5 + rng.normal(0, spread, (n, 3))) % 1.0
+    p = p.astype(np.float32)
+    p[p >= 1] = 0
+    codes, _ = orc.compute_codes(p[:, 0], p[:, 1], p[:, 2], 1)
+    perm = orc.argsort_stable(codes)
+    P = [_cuda(p[perm][:, k]) for k in range(3)]
+    tm = OctreeManager(n, node_table=True, bucket=64)
+    tm.build(P, torch.full((n,), 1.0 / n, device="cuda"), _cuda(codes[perm]))
+    f = torch.empty((n, 3), device="cuda")
+    stats = torch.zeros(4, dtype=torch.int64, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.call("cnb_forces_grouped", *(q.data_ptr() for q in P), tm.node_table.data_ptr(),
+              tm.workspace.data_ptr(), f.data_ptr(), n, 0.0, None, _lib.MAC_REF_X, 2, 4, 1.0, 0.01, 1.0, 0.0,
+              stats.data_ptr(), status.data_ptr(), int(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert int(stats[0]) == n * n
