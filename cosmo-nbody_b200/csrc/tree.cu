@@ -89,14 +89,15 @@ __device__ __forceinline__ Split split_of(const uint64_t *__restrict__ codes, I 
     return r;
 }
 
-// tree_kernels.py:60-129 build_tree, one thread per split i < n-1.
+// tree_kernels.py:60-129 build_tree, one thread per split i < n-1 (I: see split_of).
+template <typename I>
 __global__ void __launch_bounds__(256) k_build_tree(const uint64_t *__restrict__ codes,
                                                     int32_t *__restrict__ children,
                                                     int32_t *__restrict__ parents, int64_t n,
                                                     int2 *__restrict__ ranges) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n - 1;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const Split q = split_of<int64_t>(codes, i, n);
+        const Split q = split_of<I>(codes, (I)i, (I)n);
         const int64_t idx = i + n;
         children[2 * idx] = q.c0;
         children[2 * idx + 1] = q.c1;
@@ -263,126 +264,278 @@ __device__ __forceinline__ float two_sum_err(float a, float b, float s) {
     return __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
-// tree_kernels.py:131-191 compute_multipoles.  One thread per leaf; the
-// second arrival at a node (atomic counter) forms it from its two children
-// as (left + right) and climbs on.  The counter increment is an acq_rel
-// atomic: it releases the node's data and acquires the sibling's, which are
-// then read through L2.  No thread ever waits.  A climb longer
-// than the node count flags CNB_FLAG_BAD_TOPOLOGY and stops.
+// The arrays a node's values live in (n_err: compensated mode only).
+struct NodeArrays {
+    float *mass, *com, *lo, *hi;
+    float4 *err;
+};
+
 template <bool COMP>
-__global__ void __launch_bounds__(256) k_upward(const float *__restrict__ px,
-                                                const float *__restrict__ py,
-                                                const float *__restrict__ pz,
-                                                const float *__restrict__ mass,
-                                                const int32_t *__restrict__ children,
-                                                const int32_t *__restrict__ parents,
-                                                float *n_mass, float *n_com, float *n_min,
-                                                float *n_max, float *n_err, int32_t *counts,
-                                                int64_t n, int32_t *status) {
+__device__ __forceinline__ void store_node(const NodeArrays &A, int64_t v, const Acc &a) {
+    A.mass[v] = a.m;
+    A.com[3 * v] = a.cx;
+    A.com[3 * v + 1] = a.cy;
+    A.com[3 * v + 2] = a.cz;
+    A.lo[3 * v] = a.lx;
+    A.lo[3 * v + 1] = a.ly;
+    A.lo[3 * v + 2] = a.lz;
+    A.hi[3 * v] = a.hx;
+    A.hi[3 * v + 1] = a.hy;
+    A.hi[3 * v + 2] = a.hz;
+    if (COMP) A.err[v] = make_float4(a.em, a.ex, a.ey, a.ez);
+}
+
+template <bool COMP>
+__device__ __forceinline__ Acc load_node_acc(const NodeArrays &A, int64_t v) {
+    Acc b;
+    b.m = __ldcg(A.mass + v);
+    b.cx = __ldcg(A.com + 3 * v);
+    b.cy = __ldcg(A.com + 3 * v + 1);
+    b.cz = __ldcg(A.com + 3 * v + 2);
+    b.lx = __ldcg(A.lo + 3 * v);
+    b.ly = __ldcg(A.lo + 3 * v + 1);
+    b.lz = __ldcg(A.lo + 3 * v + 2);
+    b.hx = __ldcg(A.hi + 3 * v);
+    b.hy = __ldcg(A.hi + 3 * v + 1);
+    b.hz = __ldcg(A.hi + 3 * v + 2);
+    if (COMP) {
+        const float4 e = __ldcg(A.err + v);
+        b.em = e.x;
+        b.ex = e.y;
+        b.ey = e.z;
+        b.ez = e.w;
+    }
+    return b;
+}
+
+// tree_kernels.py:174-188: the parent of children L and R.
+template <bool COMP>
+__device__ __forceinline__ Acc join(const Acc &L, const Acc &R) {
+    Acc q;
+    q.m = __fadd_rn(L.m, R.m);
+    q.cx = __fadd_rn(L.cx, R.cx);
+    q.cy = __fadd_rn(L.cy, R.cy);
+    q.cz = __fadd_rn(L.cz, R.cz);
+    q.lx = pmin(L.lx, R.lx);
+    q.ly = pmin(L.ly, R.ly);
+    q.lz = pmin(L.lz, R.lz);
+    q.hx = pmax(L.hx, R.hx);
+    q.hy = pmax(L.hy, R.hy);
+    q.hz = pmax(L.hz, R.hz);
+    if (COMP) {
+        q.em = __fadd_rn(__fadd_rn(L.em, R.em), two_sum_err(L.m, R.m, q.m));
+        q.ex = __fadd_rn(__fadd_rn(L.ex, R.ex), two_sum_err(L.cx, R.cx, q.cx));
+        q.ey = __fadd_rn(__fadd_rn(L.ey, R.ey), two_sum_err(L.cy, R.cy, q.cy));
+        q.ez = __fadd_rn(__fadd_rn(L.ez, R.ez), two_sum_err(L.cz, R.cz, q.cz));
+    }
+    return q;
+}
+
+// Climbs from node curr (its values a already in the node arrays) with the
+// global counters: the second arrival at a node forms it from its two
+// children as (left + right) and climbs on.  The counter increment is an
+// acq_rel atomic: it releases the node's data and acquires the sibling's,
+// which are then read through L2.  No thread ever waits.  A climb longer than
+// the node count flags CNB_FLAG_BAD_TOPOLOGY and stops.
+template <bool COMP>
+__device__ __forceinline__ void climb_global(const NodeArrays &A, int64_t curr, int32_t p, Acc a,
+                                             const int32_t *__restrict__ children,
+                                             const int32_t *__restrict__ parents, int32_t *counts,
+                                             int64_t m_nodes, int32_t *status) {
+    for (int64_t guard = 0;; ++guard) {
+        if (guard > m_nodes) {
+            set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
+            return;
+        }
+        if (p == -1) return;
+        if (p < 0 || p >= m_nodes) {
+            set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
+            return;
+        }
+        // this level's and the next level's topology are read while the
+        // counter's atomic is in flight (they do not depend on it)
+        const int32_t l = __ldg(children + 2 * (int64_t)p), r = __ldg(children + 2 * (int64_t)p + 1);
+        const int32_t pp = __ldg(parents + p);
+        // release this node's data, acquire the sibling's: the first arrival stops
+        if (atomic_add_acq_rel(counts + p, 1) == 0) return;
+        const bool mine_left = (l == curr);
+        const int64_t s = mine_left ? r : l;
+        if ((!mine_left && r != curr) || s == curr || s < 0 || s >= m_nodes) {
+            set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
+            return;
+        }
+        const Acc b = load_node_acc<COMP>(A, s);
+        a = mine_left ? join<COMP>(a, b) : join<COMP>(b, a);
+        store_node<COMP>(A, p, a);
+        curr = p;
+        p = pp;
+    }
+}
+
+// tree_kernels.py:131-191 compute_multipoles in two launches.
+//
+// k_upward, one leaf per thread: internal node n + i lies at an end of its
+// bodies' range, so a node whose bodies are all in the block's kUpBlock
+// consecutive ones has its slot there too.  Such nodes (99 % at 128^3) are
+// formed in shared memory, with shared arrival counters, and written together,
+// consecutive addresses on consecutive threads, their counters set to the two
+// arrivals.  A node whose parent is outside the block, or whose parent saw no
+// second arrival in the block, is left for the second launch: the block lists
+// them in its part of the leaves' counters (otherwise unused and zero).
+// k_upward_rest climbs from the listed nodes with the global counters, and
+// zeroes the list.
+//
+// HBM-bound in principle (88 bytes a node: values out, topology in).  One
+// climb per leaf through global counters took 222 us at 128^3; climbing on from
+// the block inside the first launch 211 to 258 (its last climb keeps a block
+// resident); this 101 + 52.
+constexpr int kUpBlock = 512;
+
+template <bool COMP>
+constexpr int upward_smem() {
+    return (int)((COMP ? 14 : 10) * 2 * kUpBlock * sizeof(float) + 5 * kUpBlock * sizeof(int32_t));
+}
+
+template <bool COMP>
+__global__ void __launch_bounds__(kUpBlock) k_upward(const float *__restrict__ px,
+                                                     const float *__restrict__ py,
+                                                     const float *__restrict__ pz,
+                                                     const float *__restrict__ mass,
+                                                     const int32_t *__restrict__ children,
+                                                     const int32_t *__restrict__ parents,
+                                                     NodeArrays A, int32_t *counts, int64_t n,
+                                                     int32_t *status) {
+    extern __shared__ float s_val[];  // [10 or 14][2 * kUpBlock]: leaves, then internal nodes
+    constexpr int W = 2 * kUpBlock;
+    int32_t *s_cnt = reinterpret_cast<int32_t *>(s_val + (COMP ? 14 : 10) * W);  // arrivals
+    int32_t *s_who = s_cnt + kUpBlock;                                            // the first to arrive
+    int32_t *s_l = s_who + kUpBlock, *s_r = s_l + kUpBlock, *s_p = s_r + kUpBlock;  // topology
+    __shared__ int s_left;                                                        // nodes left
     const int64_t m_nodes = 2 * n - 1;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
+    const int t = threadIdx.x;
+    const int64_t b0 = blockIdx.x * (int64_t)kUpBlock, i = b0 + t;
+    const auto put = [&](int k, const Acc &a) {
+        float *v = s_val + k;
+        v[0] = a.m; v[W] = a.cx; v[2 * W] = a.cy; v[3 * W] = a.cz;
+        v[4 * W] = a.lx; v[5 * W] = a.ly; v[6 * W] = a.lz;
+        v[7 * W] = a.hx; v[8 * W] = a.hy; v[9 * W] = a.hz;
+        if (COMP) { v[10 * W] = a.em; v[11 * W] = a.ex; v[12 * W] = a.ey; v[13 * W] = a.ez; }
+    };
+    const auto get = [&](int k) {
+        const volatile float *v = s_val + k;
         Acc a;
+        a.m = v[0]; a.cx = v[W]; a.cy = v[2 * W]; a.cz = v[3 * W];
+        a.lx = v[4 * W]; a.ly = v[5 * W]; a.lz = v[6 * W];
+        a.hx = v[7 * W]; a.hy = v[8 * W]; a.hz = v[9 * W];
+        if (COMP) { a.em = v[10 * W]; a.ex = v[11 * W]; a.ey = v[12 * W]; a.ez = v[13 * W]; }
+        return a;
+    };
+    // slot of a node of the block, or -1
+    const auto slot_of = [&](int64_t v) -> int {
+        const int64_t r = v < n ? v - b0 : v - n - b0;
+        return r < 0 || r >= kUpBlock ? -1 : (int)r + (v < n ? 0 : kUpBlock);
+    };
+    s_cnt[t] = 0;
+    if (t == 0) s_left = 0;
+    const int64_t node = n + i;  // this thread's internal node
+    if (node < m_nodes) {
+        s_l[t] = __ldg(children + 2 * node);
+        s_r[t] = __ldg(children + 2 * node + 1);
+        s_p[t] = __ldg(parents + node);
+    }
+    Acc a;
+    if (i < n) {
         a.m = mass[i];
-        float x = px[i], y = py[i], z = pz[i];
+        const float x = px[i], y = py[i], z = pz[i];
         a.cx = __fmul_rn(x, a.m);
         a.cy = __fmul_rn(y, a.m);
         a.cz = __fmul_rn(z, a.m);
         a.lx = a.hx = x;
         a.ly = a.hy = y;
         a.lz = a.hz = z;
-        n_mass[i] = a.m;
-        n_com[3 * i] = a.cx;
-        n_com[3 * i + 1] = a.cy;
-        n_com[3 * i + 2] = a.cz;
-        n_min[3 * i] = x;
-        n_min[3 * i + 1] = y;
-        n_min[3 * i + 2] = z;
-        n_max[3 * i] = x;
-        n_max[3 * i + 1] = y;
-        n_max[3 * i + 2] = z;
         if (COMP) {
             a.em = 0.f;
             a.ex = __fmaf_rn(x, a.m, -a.cx);  // exact product error
             a.ey = __fmaf_rn(y, a.m, -a.cy);
             a.ez = __fmaf_rn(z, a.m, -a.cz);
-            reinterpret_cast<float4 *>(n_err)[i] = make_float4(a.em, a.ex, a.ey, a.ez);
         }
+        put(t, a);
+    }
+    __syncthreads();
+    if (i < n) {
         int64_t curr = i;
         int32_t p = parents[curr];
-        for (int64_t guard = 0;; ++guard) {
-            if (guard > m_nodes) {
-                set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
-                break;
-            }
-            if (p == -1) break;
+        for (;;) {
+            if (p == -1) break;  // the whole tree lies in the block
             if (p < 0 || p >= m_nodes) {
                 set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
-            // this level's and the next level's topology are read while the
-            // counter's atomic is in flight (they do not depend on it)
-            const int32_t l = __ldg(children + 2 * p), r = __ldg(children + 2 * p + 1);
-            const int32_t pp = __ldg(parents + p);
-            // release this node's data, acquire the sibling's: the first arrival stops
-            if (atomic_add_acq_rel(counts + p, 1) == 0) break;
+            const int ps = p < n ? -1 : slot_of(p);
+            if (ps < 0) {
+                counts[b0 + atomicAdd(&s_left, 1)] = (int32_t)curr + 1;
+                break;
+            }
+            const int pk = ps - kUpBlock;
+            const int32_t l = s_l[pk], r = s_r[pk], pp = s_p[pk];
+            __threadfence_block();
+            const int arrived = atomicAdd(s_cnt + pk, 1);
+            if (arrived != 0) {
+                __threadfence_block();
+            } else {
+                s_who[pk] = (int32_t)curr;
+                break;
+            }
             const bool mine_left = (l == curr);
-            const int32_t s = mine_left ? r : l;
-            if ((!mine_left && r != curr) || s == curr || s < 0 || s >= m_nodes) {
+            const int64_t s = mine_left ? r : l;
+            const int ss = s < 0 || s >= m_nodes ? -1 : slot_of(s);
+            // a third arrival, a parent that is not this node's, a sibling that cannot have arrived
+            if (arrived > 1 || (!mine_left && r != curr) || s == curr || ss < 0) {
                 set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
-            Acc b;
-            b.m = __ldcg(n_mass + s);
-            b.cx = __ldcg(n_com + 3 * s);
-            b.cy = __ldcg(n_com + 3 * s + 1);
-            b.cz = __ldcg(n_com + 3 * s + 2);
-            b.lx = __ldcg(n_min + 3 * s);
-            b.ly = __ldcg(n_min + 3 * s + 1);
-            b.lz = __ldcg(n_min + 3 * s + 2);
-            b.hx = __ldcg(n_max + 3 * s);
-            b.hy = __ldcg(n_max + 3 * s + 1);
-            b.hz = __ldcg(n_max + 3 * s + 2);
-            const Acc &L = mine_left ? a : b;
-            const Acc &R = mine_left ? b : a;
-            Acc q;
-            q.m = __fadd_rn(L.m, R.m);
-            q.cx = __fadd_rn(L.cx, R.cx);
-            q.cy = __fadd_rn(L.cy, R.cy);
-            q.cz = __fadd_rn(L.cz, R.cz);
-            q.lx = pmin(L.lx, R.lx);
-            q.ly = pmin(L.ly, R.ly);
-            q.lz = pmin(L.lz, R.lz);
-            q.hx = pmax(L.hx, R.hx);
-            q.hy = pmax(L.hy, R.hy);
-            q.hz = pmax(L.hz, R.hz);
-            if (COMP) {
-                float4 e = __ldcg(reinterpret_cast<const float4 *>(n_err) + s);
-                b.em = e.x;
-                b.ex = e.y;
-                b.ey = e.z;
-                b.ez = e.w;
-                q.em = __fadd_rn(__fadd_rn(L.em, R.em), two_sum_err(L.m, R.m, q.m));
-                q.ex = __fadd_rn(__fadd_rn(L.ex, R.ex), two_sum_err(L.cx, R.cx, q.cx));
-                q.ey = __fadd_rn(__fadd_rn(L.ey, R.ey), two_sum_err(L.cy, R.cy, q.cy));
-                q.ez = __fadd_rn(__fadd_rn(L.ez, R.ez), two_sum_err(L.cz, R.cz, q.cz));
-                reinterpret_cast<float4 *>(n_err)[p] = make_float4(q.em, q.ex, q.ey, q.ez);
-            }
-            n_mass[p] = q.m;
-            n_com[3 * p] = q.cx;
-            n_com[3 * p + 1] = q.cy;
-            n_com[3 * p + 2] = q.cz;
-            n_min[3 * p] = q.lx;
-            n_min[3 * p + 1] = q.ly;
-            n_min[3 * p + 2] = q.lz;
-            n_max[3 * p] = q.hx;
-            n_max[3 * p + 1] = q.hy;
-            n_max[3 * p + 2] = q.hz;
-            a = q;
+            const Acc b = get(ss);
+            a = mine_left ? join<COMP>(a, b) : join<COMP>(b, a);
+            put(ps, a);
             curr = p;
             p = pp;
         }
     }
+    __syncthreads();
+    // one array after the other, its floats on consecutive threads
+    const auto write = [&](int base, int64_t first, int64_t end, bool leaf) {
+        const int k = (int)min((int64_t)kUpBlock, end - first);  // nodes first .. first + k
+        const float *v = s_val + base;
+        if (t < k && (leaf || s_cnt[t] >= 2)) {
+            A.mass[first + t] = v[t];
+            if (COMP) A.err[first + t] = make_float4(v[10 * W + t], v[11 * W + t], v[12 * W + t], v[13 * W + t]);
+        }
+        float *out[3] = {A.com, A.lo, A.hi};
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            for (int j = t; j < 3 * k; j += kUpBlock) {
+                const int u = j / 3;
+                if (leaf || s_cnt[u] >= 2) out[q][3 * first + j] = v[(1 + 3 * q + j - 3 * u) * W + u];
+            }
+    };
+    write(0, b0, n, true);
+    write(kUpBlock, n + b0, m_nodes, false);
+    if (node < m_nodes && s_cnt[t] >= 2) counts[node] = 2;
+    if (node < m_nodes && s_cnt[t] == 1) counts[b0 + atomicAdd(&s_left, 1)] = s_who[t] + 1;
+}
+
+template <bool COMP>
+__global__ void __launch_bounds__(256) k_upward_rest(const int32_t *__restrict__ children,
+                                                     const int32_t *__restrict__ parents,
+                                                     NodeArrays A, int32_t *counts, int64_t n,
+                                                     int32_t *status) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t curr = (int64_t)counts[i] - 1;
+    if (curr < 0) return;
+    counts[i] = 0;
+    climb_global<COMP>(A, curr, parents[curr], load_node_acc<COMP>(A, curr), children, parents, counts,
+                       2 * n - 1, status);
 }
 
 // tree_kernels.py:193-214 normalize_com: inv = 1.0 / m in float64, com * inv
@@ -456,11 +609,24 @@ __global__ void k_root_store(const double *__restrict__ acc, float *n_mass, floa
     for (int k = 0; k < 3; ++k) root_out[1 + k] = c[k];
 }
 
-// tree_kernels.py:216-234 find_root.
-__global__ void k_find_root(const int32_t *__restrict__ parents, int32_t *root_idx, int64_t m) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x)
-        if (parents[i] == -1) atomicExch(root_idx, (int32_t)i);
+// tree_kernels.py:216-234 find_root.  HBM-bound: 4 bytes a node, four nodes a
+// load where the array allows it (head nodes before the first 16-byte
+// boundary, then quads, then the rest): 128^3 14 -> 5 us.
+__global__ void __launch_bounds__(256) k_find_root(const int32_t *__restrict__ parents, int32_t *root_idx,
+                                                   int64_t head, int64_t quads, int64_t m) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int4 *p4 = reinterpret_cast<const int4 *>(parents + head);
+    for (int64_t q = t; q < quads; q += (int64_t)gridDim.x * blockDim.x) {
+        const int4 v = __ldcs(p4 + q);
+        const int64_t i = head + 4 * q;
+        if (v.x == -1) atomicExch(root_idx, (int32_t)i);
+        if (v.y == -1) atomicExch(root_idx, (int32_t)i + 1);
+        if (v.z == -1) atomicExch(root_idx, (int32_t)i + 2);
+        if (v.w == -1) atomicExch(root_idx, (int32_t)i + 3);
+    }
+    if (t < head && parents[t] == -1) atomicExch(root_idx, (int32_t)t);
+    const int64_t e = head + 4 * quads + t;
+    if (e < m && t < 4 && parents[e] == -1) atomicExch(root_idx, (int32_t)e);
 }
 
 // tree_kernels.py:264-313 build_top_tree_cache: breadth-first list of the
@@ -505,25 +671,28 @@ extern "C" int cnb_reset_tree_buffers(int32_t *child, int32_t *parent, int32_t *
     return launch_status();
 }
 
+static int build_tree(const uint64_t *codes, int32_t *children, int32_t *parents, int2 *ranges,
+                      int64_t n, cudaStream_t st) {
+    if (2 * n - 1 > (int64_t)INT32_MAX) return CNB_E_TOO_LARGE;
+    if (n < 2) return CNB_OK;
+    if (n <= (int64_t)1 << 29)
+        k_build_tree<int><<<grid_for(n - 1, 256), 256, 0, st>>>(codes, children, parents, n, ranges);
+    else
+        k_build_tree<int64_t><<<grid_for(n - 1, 256), 256, 0, st>>>(codes, children, parents, n, ranges);
+    return launch_status();
+}
+
 extern "C" int cnb_build_tree(const uint64_t *codes, int32_t *children, int32_t *parents,
                               int64_t n, void *stream) {
     if (n < 0 || (n > 1 && (!codes || !children || !parents))) return CNB_E_INVALID_ARG;
-    if (2 * n - 1 > (int64_t)INT32_MAX) return CNB_E_TOO_LARGE;
-    if (n < 2) return CNB_OK;
-    k_build_tree<<<grid_for(n - 1, 256), 256, 0, as_stream(stream)>>>(codes, children, parents,
-                                                                       n, nullptr);
-    return launch_status();
+    return build_tree(codes, children, parents, nullptr, n, as_stream(stream));
 }
 
 extern "C" int cnb_build_tree_ranges(const uint64_t *codes, int32_t *children, int32_t *parents,
                                      int32_t *ranges, int64_t n, void *stream) {
     if (n < 0 || (n > 1 && (!codes || !children || !parents || !ranges))) return CNB_E_INVALID_ARG;
     if ((reinterpret_cast<uintptr_t>(ranges) & 7) != 0) return CNB_E_INVALID_ARG;
-    if (2 * n - 1 > (int64_t)INT32_MAX) return CNB_E_TOO_LARGE;
-    if (n < 2) return CNB_OK;
-    k_build_tree<<<grid_for(n - 1, 256), 256, 0, as_stream(stream)>>>(
-        codes, children, parents, n, reinterpret_cast<int2 *>(ranges));
-    return launch_status();
+    return build_tree(codes, children, parents, reinterpret_cast<int2 *>(ranges), n, as_stream(stream));
 }
 
 static int make_buckets(const int32_t *ranges, const int32_t *parents, const uint64_t *codes,
@@ -598,14 +767,24 @@ static int upward_impl(const float *px, const float *py, const float *pz, const 
                        const int32_t *children, const int32_t *parents, float *n_mass,
                        float *n_com, float *n_min, float *n_max, float *n_err, int32_t *counts,
                        int64_t n, bool comp, int32_t *status, cudaStream_t st) {
-    if (comp)
-        k_upward<true><<<grid_for(n, 256), 256, 0, st>>>(px, py, pz, mass, children, parents,
-                                                         n_mass, n_com, n_min, n_max, n_err,
-                                                         counts, n, status);
-    else
-        k_upward<false><<<grid_for(n, 256), 256, 0, st>>>(px, py, pz, mass, children, parents,
-                                                          n_mass, n_com, n_min, n_max, nullptr,
-                                                          counts, n, status);
+    const NodeArrays A{n_mass, n_com, n_min, n_max, reinterpret_cast<float4 *>(n_err)};
+    const int64_t blocks = (n + kUpBlock - 1) / kUpBlock;
+    const unsigned rest = (unsigned)((n + 255) / 256);
+    if (comp) {
+        CNB_CUDA(cudaFuncSetAttribute(k_upward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      upward_smem<true>()));
+        k_upward<true><<<(unsigned)blocks, kUpBlock, upward_smem<true>(), st>>>(
+            px, py, pz, mass, children, parents, A, counts, n, status);
+        CNB_TRY(launch_status());
+        k_upward_rest<true><<<rest, 256, 0, st>>>(children, parents, A, counts, n, status);
+    } else {
+        CNB_CUDA(cudaFuncSetAttribute(k_upward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      upward_smem<false>()));
+        k_upward<false><<<(unsigned)blocks, kUpBlock, upward_smem<false>(), st>>>(
+            px, py, pz, mass, children, parents, A, counts, n, status);
+        CNB_TRY(launch_status());
+        k_upward_rest<false><<<rest, 256, 0, st>>>(children, parents, A, counts, n, status);
+    }
     return launch_status();
 }
 
@@ -678,7 +857,11 @@ extern "C" int cnb_find_root(const int32_t *parents, int32_t *root_idx, int64_t 
                              void *stream) {
     if (n_nodes < 0 || !root_idx || (n_nodes > 0 && !parents)) return CNB_E_INVALID_ARG;
     if (n_nodes == 0) return CNB_OK;
-    k_find_root<<<grid_for(n_nodes, 256), 256, 0, as_stream(stream)>>>(parents, root_idx, n_nodes);
+    int64_t head = (16 - (int64_t)(reinterpret_cast<uintptr_t>(parents) & 15)) / 4 % 4;
+    if (head > n_nodes) head = n_nodes;
+    const int64_t quads = (n_nodes - head) / 4;
+    k_find_root<<<grid_for(quads > 0 ? quads : 1, 256, 148 * 8), 256, 0, as_stream(stream)>>>(
+        parents, root_idx, head, quads, n_nodes);
     return launch_status();
 }
 
