@@ -65,18 +65,46 @@ __device__ __forceinline__ Split split_of(const uint64_t *__restrict__ codes, I 
     const int d_next = delta_any<I>(codes, ki, i, i + 1, n);
     const I dir = d_next > d_prev ? 1 : -1;
     const int min_delta = d_next > d_prev ? d_prev : d_next;
-    I l_max = 2;
-    while (delta_any<I>(codes, ki, i, i + l_max * dir, n) > min_delta) l_max *= 2;
-    I l = 0;
-    for (I t = l_max >> 1; t >= 1; t >>= 1)  // t > 0: the reference's t // 2
-        if (delta_any<I>(codes, ki, i, i + (l + t) * dir, n) > min_delta) l += t;
+    I l_max = 2, l = 0, s = 0;
+    if (min_delta < 64) {
+        // delta(i, j) > d for d < 64 is: j exists and the keys share their first d + 1 bits
+        // (equal keys share all 64).  A mask for those bits tests that in a third of the
+        // instructions, and this search is bound by them (issue 76% busy, ALU 64%, DRAM 4%):
+        // 2 097 152 keys 57 -> 47 us, with buckets 65 -> 53, 16 777 216 with buckets 453 -> 373.
+        const auto shares = [&](I j, uint64_t bits) {
+            if constexpr (sizeof(I) == 4) {
+                if ((unsigned)j >= (unsigned)n) return false;
+            } else {
+                if (j < 0 || j >= n) return false;
+            }
+            return ((__ldg(codes + j) ^ ki) & bits) == 0ull;
+        };
+        const auto first_bits = [](int d) { return ~(0x7fffffffffffffffull >> d); };  // d + 1 of them
+        const uint64_t bits = min_delta < 0 ? 0ull : first_bits(min_delta);
+        while (shares(i + l_max * dir, bits)) l_max *= 2;
+        for (I t = l_max >> 1; t >= 1; t >>= 1)  // t > 0: the reference's t // 2
+            if (shares(i + (l + t) * dir, bits)) l += t;
+    } else {
+        while (delta_any<I>(codes, ki, i, i + l_max * dir, n) > min_delta) l_max *= 2;
+        for (I t = l_max >> 1; t >= 1; t >>= 1)
+            if (delta_any<I>(codes, ki, i, i + (l + t) * dir, n) > min_delta) l += t;
+    }
     const I j = i + l * dir;
     const int delta_node = delta_any<I>(codes, ki, i, j, n);
-    I s = 0;
-    for (I t = l; t > 0;) {
-        I step = (t + 1) >> 1;
-        if (delta_any<I>(codes, ki, i, i + (s + step) * dir, n) > delta_node) s += step;
-        t -= step;
+    if (delta_node < 64) {
+        // j and so every index between lies in the array
+        const uint64_t bits = ~(0x7fffffffffffffffull >> delta_node);
+        for (I t = l; t > 0;) {
+            I step = (t + 1) >> 1;
+            if (((__ldg(codes + i + (s + step) * dir) ^ ki) & bits) == 0ull) s += step;
+            t -= step;
+        }
+    } else {
+        for (I t = l; t > 0;) {
+            I step = (t + 1) >> 1;
+            if (delta_any<I>(codes, ki, i, i + (s + step) * dir, n) > delta_node) s += step;
+            t -= step;
+        }
     }
     Split r;
     I gamma = i + s * dir;
