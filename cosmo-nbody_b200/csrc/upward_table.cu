@@ -219,14 +219,22 @@ __global__ void __launch_bounds__(256) k_upward_table(
 // the right child by its first), so the bucket's children are one coalesced
 // read.  The warp checks that they form a tree over the bucket's bodies
 // (every body and node but the root has exactly one parent), loads the
-// leaves, and then forms, round after round, every node whose two children
-// are ready; each lane owns at most two of the bucket's nodes, no lane waits
-// on another and no atomic is needed; the records are written afterwards,
-// consecutive nodes on consecutive lanes.  Every node is formed as
-// (left + right) of its children: the table is bit-identical to the
-// one-phase pass.  After every 32 buckets a warp climbs on above their
-// roots, one lane each, with the global counters (the first arrival at a
-// node stops, as in the one-phase pass).
+// leaves, and then forms, round after round, nodes whose two children are
+// ready: which are is two words that every lane knows.  A lane owns at most
+// two of the bucket's nodes and forms one a round; no lane waits on another
+// and no atomic is needed; the records are written afterwards, consecutive
+// nodes on consecutive lanes.  Every node is formed as (left + right) of its
+// children: the table is bit-identical to the one-phase pass.  After every 32
+// buckets a warp climbs on above their roots, one lane each, with the global
+// counters (the first arrival at a node stops, as in the one-phase pass).
+//
+// Bound by the instructions of the rounds (issue 61% busy, DRAM 31%), with
+// the climb's chain of fences and atomics, 1.7 us a level, behind them.  The
+// links checked as bits instead of by shared-memory exchanges, the ready flags
+// in registers and 40 bytes a slot instead of 48 took the registers from 94 to
+// 72 and 20 warps an SM to 28: 2 097 152 bodies 134 -> 117 us, 16 777 216 902 ->
+// 736, 300 007 with moments 60 -> 52.  Measured without a gain: 32 or 24 warps
+// an SM, one 256-bit store a record.
 constexpr int kUpSlots = 64;  // leaves of a bucket; its internal nodes use as many slots
 constexpr int kUpWarps = 4;
 
@@ -255,19 +263,22 @@ __device__ __forceinline__ void climb_roots(int64_t root, const int2 *__restrict
     __syncwarp();
 }
 
+__device__ __forceinline__ uint64_t or_of_lanes(uint64_t v) {
+    return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32)) << 32 |
+           __reduce_or_sync(0xffffffffu, (uint32_t)v);
+}
+
 template <bool QUAD>
-__global__ void __launch_bounds__(kUpWarps * 32) k_upward_buckets(
+__global__ void __launch_bounds__(kUpWarps * 32, QUAD ? 6 : 7) k_upward_buckets(
     const float *__restrict__ px, const float *__restrict__ py, const float *__restrict__ pz,
     const float *__restrict__ mass, const int2 *__restrict__ children,
     const int32_t *__restrict__ parents, const int32_t *__restrict__ ws, int32_t *counts,
     float4 *sums, float4 *rec, float4 *aabb, float4 *quad, int64_t n, int32_t *status) {
-    // slot k < kUpSlots: leaf lo + k; slot kUpSlots + k: internal node n + lo + k
-    __shared__ float4 s_sum[kUpWarps][2 * kUpSlots], s_lo[kUpWarps][2 * kUpSlots],
-        s_hi[kUpWarps][2 * kUpSlots];
-    __shared__ float4 s_qa[QUAD ? kUpWarps : 1][QUAD ? 2 * kUpSlots : 1],
-        s_qb[QUAD ? kUpWarps : 1][QUAD ? 2 * kUpSlots : 1];
-    __shared__ int s_par[kUpWarps][2 * kUpSlots];  // parent (internal index) of each slot
-    __shared__ int s_rdy[kUpWarps][2 * kUpSlots];  // the slot's data is in shared memory
+    // slot k < kUpSlots: leaf lo + k; slot kUpSlots + k: internal node n + lo + off + k
+    __shared__ float4 s_sum[kUpWarps][2 * kUpSlots], s_box[kUpWarps][2 * kUpSlots];
+    __shared__ float2 s_top[kUpWarps][2 * kUpSlots];  // box: (lo.xyz, hi.x) and (hi.y, hi.z)
+    __shared__ float4 s_qa[QUAD ? kUpWarps : 1][QUAD ? kUpSlots : 1];  // internal nodes only
+    __shared__ float2 s_qb[QUAD ? kUpWarps : 1][QUAD ? kUpSlots : 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nb = ws[0];
     const int4 *buckets = reinterpret_cast<const int4 *>(ws + 4);
@@ -289,7 +300,6 @@ __global__ void __launch_bounds__(kUpWarps * 32) k_upward_buckets(
         const int lo_b = bk.x, count = bk.y;
         const int64_t root = bk.z;
         const int off = (count > 1 && root == n + lo_b + count - 1) ? 1 : 0;  // first internal slot
-        const int root_slot = count == 1 ? 0 : kUpSlots + (int)(root - n - lo_b);
         if (count > kUpSlots) {
             if (lane == 0) set_flag(status, CNB_FLAG_LIST_OVERFLOW);
             continue;
@@ -314,42 +324,41 @@ __global__ void __launch_bounds__(kUpWarps * 32) k_upward_buckets(
             own[h] = off + k < off + count - 1;
             chn[h] = own[h] ? __ldg(children + n + lo_b + off + k) : make_int2(-1, -1);
         }
-        for (int k = lane; k < 2 * kUpSlots; k += 32) {
-            s_par[w][k] = -1;
-            s_rdy[w][k] = k < count;  // the leaves are ready once stored
-        }
-        __syncwarp();
-        // this lane's internal nodes: slots kUpSlots + off + lane (+ 32), children at a[][]
-        int a[2][2];
+        // this lane's internal nodes, bits lane and lane + 32: the slots of their children
+        // and, as bits, the internal nodes among those
+        const int n_int = count - 1;
+        const uint64_t all_int = (1ull << n_int) - 1ull;
+        int kid[2];
+        uint64_t need[2], leaves = 0ull;
         bool bad = false;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int k = off + lane + 32 * h;
-            a[h][0] = a[h][1] = 0;
+            kid[h] = 0;
+            need[h] = 0ull;
             if (!own[h]) continue;
-            bool ok = true;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const int64_t v = c == 0 ? chn[h].x : chn[h].y;
-                const int64_t r = v < n ? v - lo_b : v - n - lo_b;
-                ok = ok && v >= 0 && (v < n ? r >= 0 && r < count : r >= off && r < off + count - 1);
-                a[h][c] = ok ? (v < n ? (int)r : kUpSlots + (int)r) : 0;
+                const int64_t r = v < n ? v - lo_b : v - n - lo_b - off;
+                if (v >= 0 && r >= 0 && r < (v < n ? count : n_int)) {
+                    if (v < n) leaves |= 1ull << r;
+                    else need[h] |= 1ull << r;
+                    kid[h] |= ((v < n ? 0 : kUpSlots) + (int)r) << (8 * c);
+                } else {
+                    bad = true;
+                }
             }
-            if (ok && a[h][0] != a[h][1])
-                bad |= (atomicExch(&s_par[w][a[h][0]], k) != -1) |
-                       (atomicExch(&s_par[w][a[h][1]], k) != -1);
-            else
-                bad = true;
         }
-        __syncwarp();
-        // a tree: every slot but the root has exactly one parent, the root none
-        for (int k = lane; k < count; k += 32) bad |= (s_par[w][k] < 0) != (k == root_slot);
-        for (int k = off + lane; k < off + count - 1; k += 32)
-            bad |= (s_par[w][kUpSlots + k] < 0) != (kUpSlots + k == root_slot);
+        // a tree: the 2 n_int links of the n_int nodes reach all of the 2 n_int other slots
+        // than the root's, so each exactly once
+        const uint64_t root_bit = n_int == 0 ? 0ull : off ? 1ull << (n_int - 1) : 1ull;
+        const uint64_t lw = or_of_lanes(leaves), nw = or_of_lanes(need[0] | need[1]);
+        bad |= n_int > 0 && (lw != (all_int << 1 | 1ull) || nw != (all_int ^ root_bit));
         if (__any_sync(0xffffffffu, bad)) {
             if (lane == 0) set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
             continue;
         }
+        __syncwarp();  // the last bucket's records have been read
         // the leaves
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -363,47 +372,53 @@ __global__ void __launch_bounds__(kUpWarps * 32) k_upward_buckets(
             if (i == root) sums[i] = sv;
             store_record(rec, aabb, i, sv, lv, lv, -1, -1);
             s_sum[w][k] = sv;
-            s_lo[w][k] = lv;
-            s_hi[w][k] = lv;
-            if (QUAD) s_qa[w][k] = s_qb[w][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            s_box[w][k] = make_float4(x, y, z, x);
+            s_top[w][k] = make_float2(y, z);
         }
         __syncwarp();
-        // the internal nodes, round by round (a round forms every node whose
-        // children are ready; a valid bucket needs at most count - 1 rounds)
-        bool done[2] = {!own[0], !own[1]};
-        for (int round = 0; round < count; ++round) {
-            bool formed[2] = {false, false};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (done[h] || !s_rdy[w][a[h][0]] || !s_rdy[w][a[h][1]]) continue;
-                const int l = a[h][0], r = a[h][1], ns = kUpSlots + off + lane + 32 * h;
+        // the internal nodes, round by round (a valid bucket needs at most n_int rounds; a
+        // cycle leaves some of them unformed and a round without any)
+        uint64_t done = 0ull;
+        bool left0 = own[0], left1 = own[1];
+        while (done != all_int) {
+            const bool r0 = left0 && (need[0] & ~done) == 0ull;
+            const bool r1 = !r0 && left1 && (need[1] & ~done) == 0ull;
+            left0 = left0 && !r0;
+            left1 = left1 && !r1;
+            if (r0 || r1) {
+                const int k = r0 ? kid[0] : kid[1], l = k & 255, r = k >> 8;
+                const int ns = kUpSlots + lane + (r0 ? 0 : 32);
                 const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 qs, qlo, qhi, na = zero, nb = zero;
-                combine<QUAD>(s_sum[w][l], s_lo[w][l], s_hi[w][l], QUAD ? s_qa[w][l] : zero,
-                              QUAD ? s_qb[w][l] : zero, s_sum[w][r], s_lo[w][r], s_hi[w][r],
-                              QUAD ? s_qa[w][r] : zero, QUAD ? s_qb[w][r] : zero, qs, qlo, qhi, na,
-                              nb);
+                const float4 lb = s_box[w][l], rb = s_box[w][r];
+                const float2 lt = s_top[w][l], rt = s_top[w][r];
+                float4 la = zero, lq = zero, ra = zero, rq = zero;
+                if (QUAD && l >= kUpSlots) {
+                    la = s_qa[w][l - kUpSlots];
+                    const float2 q = s_qb[w][l - kUpSlots];
+                    lq = make_float4(q.x, q.y, 0.f, 0.f);
+                }
+                if (QUAD && r >= kUpSlots) {
+                    ra = s_qa[w][r - kUpSlots];
+                    const float2 q = s_qb[w][r - kUpSlots];
+                    rq = make_float4(q.x, q.y, 0.f, 0.f);
+                }
+                float4 qs, qlo, qhi, na = zero, nb4 = zero;
+                combine<QUAD>(s_sum[w][l], lb, make_float4(lb.w, lt.x, lt.y, 0.f), la, lq, s_sum[w][r],
+                              rb, make_float4(rb.w, rt.x, rt.y, 0.f), ra, rq, qs, qlo, qhi, na, nb4);
                 s_sum[w][ns] = qs;
-                s_lo[w][ns] = qlo;
-                s_hi[w][ns] = qhi;
+                s_box[w][ns] = make_float4(qlo.x, qlo.y, qlo.z, qhi.x);
+                s_top[w][ns] = make_float2(qhi.y, qhi.z);
                 if (QUAD) {
-                    s_qa[w][ns] = na;
-                    s_qb[w][ns] = nb;
+                    s_qa[w][ns - kUpSlots] = na;
+                    s_qb[w][ns - kUpSlots] = make_float2(nb4.x, nb4.y);
                 }
-                formed[h] = true;
             }
-            __syncwarp();  // the data of this round's nodes before their flags
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                if (formed[h]) {
-                    s_rdy[w][kUpSlots + off + lane + 32 * h] = 1;
-                    done[h] = true;
-                }
+            const uint32_t f0 = __ballot_sync(0xffffffffu, r0), f1 = __ballot_sync(0xffffffffu, r1);
+            if ((f0 | f1) == 0u) break;
+            done |= (uint64_t)f1 << 32 | f0;
             __syncwarp();
-            if (!__any_sync(0xffffffffu, !(done[0] && done[1]))) break;
         }
-        // a cycle among the internal nodes leaves some of them unformed
-        if (__any_sync(0xffffffffu, !(done[0] && done[1]))) {
+        if (done != all_int) {
             if (lane == 0) set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
             continue;
         }
@@ -411,12 +426,19 @@ __global__ void __launch_bounds__(kUpWarps * 32) k_upward_buckets(
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (!own[h]) continue;
-            const int k = off + lane + 32 * h, ns = kUpSlots + k;
-            const int64_t p = n + lo_b + k;
-            write_node<QUAD>(p, s_sum[w][ns], s_lo[w][ns], s_hi[w][ns],
-                             QUAD ? s_qa[w][ns] : make_float4(0.f, 0.f, 0.f, 0.f),
-                             QUAD ? s_qb[w][ns] : make_float4(0.f, 0.f, 0.f, 0.f), chn[h], sums,
-                             rec, aabb, quad, p == root);
+            const int k = lane + 32 * h, ns = kUpSlots + k;
+            const int64_t p = n + lo_b + off + k;
+            const float4 bx = s_box[w][ns];
+            const float2 tp = s_top[w][ns];
+            float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb4 = na;
+            if (QUAD) {
+                na = s_qa[w][k];
+                const float2 q = s_qb[w][k];
+                nb4 = make_float4(q.x, q.y, 0.f, 0.f);
+            }
+            write_node<QUAD>(p, s_sum[w][ns], make_float4(bx.x, bx.y, bx.z, 0.f),
+                             make_float4(bx.w, tp.x, tp.y, 0.f), na, nb4, chn[h], sums, rec, aabb,
+                             quad, p == root);
         }
         if (lane == (t & 31)) my_root = root;
     }
