@@ -32,9 +32,8 @@ struct cnb_ctx {
 
 namespace cnb {
 // tiles and the bound on out-of-place keys of the near-sorted path
-constexpr int kNearThreads = 512;
-constexpr int kNearItems = 8;
-constexpr int kNearTile = kNearThreads * kNearItems;  // 4096 keys
+constexpr int kNearMinThreads = 128;                  // of a tile's block at the smallest
+constexpr int kNearItems = 8;                         // keys a thread
 constexpr int kNearCap = 2048;                        // at most this many keys leave their run
 int64_t near_bytes(int64_t n_max);
 int sort_pairs_near(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,

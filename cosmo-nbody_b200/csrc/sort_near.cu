@@ -7,7 +7,7 @@
 // except in a few places.  The path takes out a set S of keys such that the
 // rest R ascends, sorts S, and merges S back into R.  The result is exactly
 // the stable argsort (ties by index), the same as the full radix sort's.
-// Four kernels over 4096-key tiles; the last block of each of the first three
+// Four kernels over tiles of 1024, 2048 or 4096 keys (see sort_pairs_near); the last block of each of the first three
 // to finish (a completion counter, no waiting) does the step that needs every
 // tile's result:
 //   k_near_mark    a tile whose keys ascend, together with the key before and
@@ -39,6 +39,12 @@
 //                  key in its range is a shifted copy.
 // Order everywhere is (key, index) lexicographic, so equal keys keep their
 // input order.
+//
+// Bound by latency: chains of block scans in the tiles that are not clean and the
+// serial steps of the last blocks.  Tiles sized by n, no compaction before the
+// first marking round, k_near_take with a warp per tile instead of a block and
+// warp barriers in the network's short distances: 32 768 keys 40.8 -> 30.5 us,
+// 300 007 49.0 -> 40.6, 2 097 152 clustered 96.6 -> 77.3, 16 777 216 203 -> 172.
 #include "ctx.cuh"
 
 namespace cnb {
@@ -46,24 +52,33 @@ namespace cnb {
 namespace {
 
 constexpr int kNearHalo = 128;                         // keys either side of a tile
-constexpr int kNearWin = kNearTile + 2 * kNearHalo;    // 4352
-constexpr int kNearWinItems = (kNearWin + kNearThreads - 1) / kNearThreads;
 constexpr int kNearMaxDescents = 256;  // more descents in one window: give up
 constexpr int kNearRounds = 32;        // marking rounds before giving up
 constexpr int kNearReach = 256;        // keys one descent looks at on either side
-constexpr int kNearWords = kNearTile / 32;
-constexpr size_t kNearMarkSmem = (size_t)kNearWin * (sizeof(uint64_t) + sizeof(uint16_t) + 1);
-constexpr size_t kNearPlaceSmem = (size_t)kNearTile * (sizeof(uint64_t) + sizeof(uint32_t));
 constexpr uint32_t kNone = 0xffffffffu;
-static_assert(kNearWin < 65536, "window positions are 16-bit");
-static_assert(kNearItems == 8 && kNearTile % 32 == 0, "eight keys per thread, one byte of a word");
+static_assert(kNearItems == 8, "eight keys per thread, one byte of a word");
+
+constexpr int kNearTakeThreads = 512;  // of k_near_take: its last block sorts S
+constexpr int kNearTakeTiles = kNearTakeThreads / 32;
+
+// a tile of NT threads
+template <int NT>
+struct NearTile {
+    static constexpr int keys = NT * kNearItems;
+    static constexpr int words = keys / 32;
+    static constexpr int win = keys + 2 * kNearHalo;
+    static constexpr int win_items = (win + NT - 1) / NT;
+    static constexpr size_t mark_smem = (size_t)win * (sizeof(uint64_t) + sizeof(uint16_t) + 1);
+    static constexpr size_t place_smem = (size_t)keys * (sizeof(uint64_t) + sizeof(uint32_t));
+    static_assert(win < 65536, "window positions are 16-bit");
+};
 
 struct NearWs {
     int32_t *ctl;  // [0] give up, [1] near path taken, [2] |S|, [3..5] blocks done per kernel,
                    // [6] the persistent full sort's barrier arrivals
     uint64_t *umax, *umin, *pmax, *smin, *rkey;  // per tile
     uint32_t *scnt, *soff, *rpos, *dirty, *tlo;  // per tile (soff, tlo: tiles + 1)
-    uint32_t *bits;                              // per tile kNearWords words
+    uint32_t *bits;                              // per key one bit
     uint64_t *s_key, *ss_key;                    // kNearCap
     uint32_t *s_pos, *ss_pos;                    // kNearCap
 };
@@ -91,7 +106,7 @@ int64_t near_layout(void *base, int64_t nt, NearWs *w) {
     v.rpos = reinterpret_cast<uint32_t *>(take(nt * 4));
     v.dirty = reinterpret_cast<uint32_t *>(take(nt * 4));
     v.tlo = reinterpret_cast<uint32_t *>(take((nt + 1) * 4));
-    v.bits = reinterpret_cast<uint32_t *>(take(nt * kNearWords * 4));
+    v.bits = reinterpret_cast<uint32_t *>(take(nt * NearTile<kNearMinThreads>::words * 4));
     v.s_key = reinterpret_cast<uint64_t *>(take(kNearCap * 8));
     v.ss_key = reinterpret_cast<uint64_t *>(take(kNearCap * 8));
     v.s_pos = reinterpret_cast<uint32_t *>(take(kNearCap * 4));
@@ -170,43 +185,46 @@ __device__ __forceinline__ bool last_block(int32_t *counter, int *s_flag) {
 __device__ __forceinline__ int32_t ld_flag(const int32_t *p) { return *(volatile const int32_t *)p; }
 
 // The marking of a tile with a descent (block-uniform control flow).
+template <int NT>
 __device__ void mark_window(const uint64_t *__restrict__ keys, int64_t n, int64_t t, NearWs &w,
                             unsigned char *smem, uint32_t *wsum, int *s_desc, int *s_u,
                             unsigned long long *s_max, unsigned long long *s_min) {
     uint64_t *sk = reinterpret_cast<uint64_t *>(smem);
-    uint16_t *ci = reinterpret_cast<uint16_t *>(smem + kNearWin * sizeof(uint64_t));
-    uint8_t *mk = smem + kNearWin * (sizeof(uint64_t) + sizeof(uint16_t));
-    const int64_t base = t * kNearTile;
+    uint16_t *ci = reinterpret_cast<uint16_t *>(smem + NearTile<NT>::win * sizeof(uint64_t));
+    uint8_t *mk = smem + NearTile<NT>::win * (sizeof(uint64_t) + sizeof(uint16_t));
+    const int64_t base = t * NearTile<NT>::keys;
     const int64_t lo = base - kNearHalo > 0 ? base - kNearHalo : 0;
-    const int64_t hi = base + kNearTile + kNearHalo < n ? base + kNearTile + kNearHalo : n;
+    const int64_t hi = base + NearTile<NT>::keys + kNearHalo < n ? base + NearTile<NT>::keys + kNearHalo : n;
     const int wn = (int)(hi - lo);
     const int own0 = (int)(base - lo);
-    const int own_n = (int)(n - base < kNearTile ? n - base : kNearTile);
-    uint32_t *tile_bits = w.bits + t * kNearWords;
+    const int own_n = (int)(n - base < NearTile<NT>::keys ? n - base : NearTile<NT>::keys);
+    uint32_t *tile_bits = w.bits + t * NearTile<NT>::words;
     if (threadIdx.x == 0) {
         *s_desc = 0;
+        *s_u = wn;
         *s_max = 0ull;
         *s_min = ~0ull;
     }
     {
-        uint64_t v[kNearWinItems];
+        uint64_t v[NearTile<NT>::win_items];
 #pragma unroll
-        for (int q = 0; q < kNearWinItems; ++q) {
-            const int j = threadIdx.x + q * kNearThreads;
+        for (int q = 0; q < NearTile<NT>::win_items; ++q) {
+            const int j = threadIdx.x + q * NT;
             v[q] = j < wn ? __ldg(keys + lo + j) : 0ull;
         }
 #pragma unroll
-        for (int q = 0; q < kNearWinItems; ++q) {
-            const int j = threadIdx.x + q * kNearThreads;
+        for (int q = 0; q < NearTile<NT>::win_items; ++q) {
+            const int j = threadIdx.x + q * NT;
             if (j < wn) {
                 sk[j] = v[q];
                 mk[j] = 0;
+                ci[j] = (uint16_t)j;
             }
         }
     }
     __syncthreads();
     int desc = 0;
-    for (int j = threadIdx.x; j + 1 < wn; j += kNearThreads) desc += sk[j] > sk[j + 1];
+    for (int j = threadIdx.x; j + 1 < wn; j += NT) desc += sk[j] > sk[j + 1];
     if (desc) atomicAdd(s_desc, desc);
     __syncthreads();
     if (*s_desc > kNearMaxDescents) {
@@ -215,25 +233,28 @@ __device__ void mark_window(const uint64_t *__restrict__ keys, int64_t n, int64_
     }
     bool converged = false;
     for (int r = 0; r < kNearRounds; ++r) {
-        // the unmarked window positions in order, a contiguous chunk per thread
-        const int c0 = threadIdx.x * kNearWinItems;
-        uint32_t cnt = 0;
+        // the unmarked window positions in order, a contiguous chunk per thread (every
+        // position before the first round)
+        if (r > 0) {
+            const int c0 = threadIdx.x * NearTile<NT>::win_items;
+            uint32_t cnt = 0;
 #pragma unroll
-        for (int k = 0; k < kNearWinItems; ++k) {
-            const int j = c0 + k;
-            cnt += (j < wn && !mk[j]);
-        }
-        uint32_t off = near_exsum<kNearThreads>(cnt, wsum);
+            for (int k = 0; k < NearTile<NT>::win_items; ++k) {
+                const int j = c0 + k;
+                cnt += (j < wn && !mk[j]);
+            }
+            uint32_t off = near_exsum<NT>(cnt, wsum);
 #pragma unroll
-        for (int k = 0; k < kNearWinItems; ++k) {
-            const int j = c0 + k;
-            if (j < wn && !mk[j]) ci[off++] = (uint16_t)j;
+            for (int k = 0; k < NearTile<NT>::win_items; ++k) {
+                const int j = c0 + k;
+                if (j < wn && !mk[j]) ci[off++] = (uint16_t)j;
+            }
+            if (threadIdx.x == NT - 1) *s_u = (int)off;
+            __syncthreads();
         }
-        if (threadIdx.x == kNearThreads - 1) *s_u = (int)off;
-        __syncthreads();
         const int U = *s_u;
         int changed = 0;
-        for (int c = threadIdx.x; c + 1 < U; c += kNearThreads) {
+        for (int c = threadIdx.x; c + 1 < U; c += NT) {
             const uint64_t a = sk[ci[c]], b = sk[ci[c + 1]];
             if (a > b) {
                 // the keys after the descent that are below a, and the keys
@@ -268,7 +289,7 @@ __device__ void mark_window(const uint64_t *__restrict__ keys, int64_t n, int64_
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long vmax = 0ull, vmin = ~0ull;
-    for (int q = warp; q < kNearWords; q += kNearThreads / 32) {
+    for (int q = warp; q < NearTile<NT>::words; q += NT / 32) {
         const int o = q * 32 + lane;
         const bool own = o < own_n;
         const bool m = own && mk[own0 + o];
@@ -290,17 +311,18 @@ __device__ void mark_window(const uint64_t *__restrict__ keys, int64_t n, int64_
     }
 }
 
-__global__ void __launch_bounds__(kNearThreads) k_near_mark(const uint64_t *__restrict__ keys,
+template <int NT>
+__global__ void __launch_bounds__(NT) k_near_mark(const uint64_t *__restrict__ keys,
                                                             int64_t n, int64_t nt, NearWs w) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ uint32_t wsum[kNearThreads / 32];
-    __shared__ uint64_t wtot[kNearThreads / 32];
+    __shared__ uint32_t wsum[NT / 32];
+    __shared__ uint64_t wtot[NT / 32];
     __shared__ int s_desc, s_u, s_last;
     __shared__ unsigned long long s_max, s_min;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t t = blockIdx.x;
-    const int64_t base = t * kNearTile;
-    const int own_n = (int)(n - base < kNearTile ? n - base : kNearTile);
+    const int64_t base = t * NearTile<NT>::keys;
+    const int own_n = (int)(n - base < NearTile<NT>::keys ? n - base : NearTile<NT>::keys);
     // clean test: the tile's keys, the key before it and the key after it
     // ascend (rows of 32 keys per warp, coalesced)
     uint64_t k[kNearItems];
@@ -327,8 +349,8 @@ __global__ void __launch_bounds__(kNearThreads) k_near_mark(const uint64_t *__re
     }
     if (threadIdx.x == 0 && base > 0 && __ldg(keys + base - 1) > k[0]) desc = true;
     if (!__syncthreads_or(desc)) {
-        uint32_t *tile_bits = w.bits + t * kNearWords;
-        if (threadIdx.x < kNearWords) tile_bits[threadIdx.x] = 0u;
+        uint32_t *tile_bits = w.bits + t * NearTile<NT>::words;
+        if (threadIdx.x < NearTile<NT>::words) tile_bits[threadIdx.x] = 0u;
         if (threadIdx.x == 0) {
             w.umin[t] = k[0];
             w.dirty[t] = 0u;
@@ -337,11 +359,11 @@ __global__ void __launch_bounds__(kNearThreads) k_near_mark(const uint64_t *__re
         for (int r = 0; r < kNearItems; ++r)
             if (warp * 256 + r * 32 + lane == own_n - 1) w.umax[t] = k[r];
     } else {
-        mark_window(keys, n, t, w, smem, wsum, &s_desc, &s_u, &s_max, &s_min);
+        mark_window<NT>(keys, n, t, w, smem, wsum, &s_desc, &s_u, &s_max, &s_min);
     }
     if (!last_block(w.ctl + 3, &s_last) || ld_flag(w.ctl)) return;
     // per tile: max of the unmarked keys of the tiles before, min of those after
-    const int64_t per = (nt + kNearThreads - 1) / kNearThreads;
+    const int64_t per = (nt + NT - 1) / NT;
     const int64_t a = (int64_t)threadIdx.x * per;
     const int64_t b = a + per < nt ? a + per : nt;
     uint64_t mx = 0ull, mn = ~0ull;
@@ -350,13 +372,13 @@ __global__ void __launch_bounds__(kNearThreads) k_near_mark(const uint64_t *__re
         mx = u > mx ? u : mx;
         mn = v < mn ? v : mn;
     }
-    uint64_t run = near_exscan64<kNearThreads, true>(mx, wtot);
+    uint64_t run = near_exscan64<NT, true>(mx, wtot);
     for (int64_t i = a; i < b; ++i) {
         w.pmax[i] = run;
         const uint64_t u = __ldcg(w.umax + i);
         run = u > run ? u : run;
     }
-    run = near_exscan64<kNearThreads, false>(mn, wtot);
+    run = near_exscan64<NT, false>(mn, wtot);
     for (int64_t i = b - 1; i >= a; --i) {
         w.smin[i] = run;
         const uint64_t v = __ldcg(w.umin + i);
@@ -364,18 +386,19 @@ __global__ void __launch_bounds__(kNearThreads) k_near_mark(const uint64_t *__re
     }
 }
 
-__global__ void __launch_bounds__(kNearThreads) k_near_filter(const uint64_t *__restrict__ keys,
+template <int NT>
+__global__ void __launch_bounds__(NT) k_near_filter(const uint64_t *__restrict__ keys,
                                                               int64_t n, int64_t nt, NearWs w,
                                                               unsigned long long *stats,
                                                               cudaGraphConditionalHandle cond,
                                                               bool use_cond) {
-    __shared__ uint64_t wtot[kNearThreads / 32];
-    __shared__ uint32_t wsum[kNearThreads / 32];
+    __shared__ uint64_t wtot[NT / 32];
+    __shared__ uint32_t wsum[NT / 32];
     __shared__ int s_first, s_last;
     if (ld_flag(w.ctl)) return;  // gave up: the full sort runs
     const int64_t t = blockIdx.x;
-    const int64_t base = t * kNearTile;
-    const int own_n = (int)(n - base < kNearTile ? n - base : kNearTile);
+    const int64_t base = t * NearTile<NT>::keys;
+    const int own_n = (int)(n - base < NearTile<NT>::keys ? n - base : NearTile<NT>::keys);
     const uint64_t tmin = w.umin[t], tmax = w.umax[t];
     if (!w.dirty[t] && w.pmax[t] <= tmin && w.smin[t] >= tmax) {
         // clean, and within the keys around it: all of it is R
@@ -386,8 +409,8 @@ __global__ void __launch_bounds__(kNearThreads) k_near_filter(const uint64_t *__
         }
     } else {
         const int j0 = threadIdx.x * kNearItems;
-        uint32_t *tile_bits = w.bits + t * kNearWords;
-        if (threadIdx.x == 0) s_first = kNearTile;
+        uint32_t *tile_bits = w.bits + t * NearTile<NT>::words;
+        if (threadIdx.x == 0) s_first = NearTile<NT>::keys;
         const uint32_t marks = my_byte(tile_bits);
         uint64_t k[kNearItems];
         uint64_t hmax = 0ull, hmin = ~0ull;
@@ -400,8 +423,8 @@ __global__ void __launch_bounds__(kNearThreads) k_near_filter(const uint64_t *__
                 hmin = k[q] < hmin ? k[q] : hmin;
             }
         }
-        uint64_t pre = near_exscan64<kNearThreads, true>(hmax, wtot);
-        uint64_t suf = near_exscan64<kNearThreads, false>(hmin, wtot);
+        uint64_t pre = near_exscan64<NT, true>(hmax, wtot);
+        uint64_t suf = near_exscan64<NT, false>(hmin, wtot);
         {
             const uint64_t p = w.pmax[t], s = w.smin[t];
             pre = p > pre ? p : pre;
@@ -429,17 +452,17 @@ __global__ void __launch_bounds__(kNearThreads) k_near_filter(const uint64_t *__
         word |= __shfl_xor_sync(0xffffffffu, word, 1);
         word |= __shfl_xor_sync(0xffffffffu, word, 2);
         if ((threadIdx.x & 3) == 0) tile_bits[j0 >> 5] = word;
-        int first = kNearTile;
+        int first = NearTile<NT>::keys;
 #pragma unroll
         for (int q = kNearItems - 1; q >= 0; --q)
             if (j0 + q < own_n && !((sbits >> q) & 1u)) first = j0 + q;
-        if (first < kNearTile) atomicMin(&s_first, first);
+        if (first < NearTile<NT>::keys) atomicMin(&s_first, first);
         const uint32_t cnt = (uint32_t)__popc(sbits);
-        const uint32_t ex = near_exsum<kNearThreads>(cnt, wsum);
-        if (threadIdx.x == kNearThreads - 1) {
+        const uint32_t ex = near_exsum<NT>(cnt, wsum);
+        if (threadIdx.x == NT - 1) {
             w.scnt[t] = ex + cnt;
             const int f = s_first;
-            if (f < kNearTile) {
+            if (f < NearTile<NT>::keys) {
                 w.rkey[t] = __ldg(keys + base + f);
                 w.rpos[t] = (uint32_t)(base + f);
             } else {
@@ -450,17 +473,17 @@ __global__ void __launch_bounds__(kNearThreads) k_near_filter(const uint64_t *__
     }
     if (!last_block(w.ctl + 4, &s_last)) return;
     // offsets of S per tile, and the choice of path
-    const int64_t per = (nt + kNearThreads - 1) / kNearThreads;
+    const int64_t per = (nt + NT - 1) / NT;
     const int64_t a = (int64_t)threadIdx.x * per;
     const int64_t b = a + per < nt ? a + per : nt;
     uint32_t sum = 0;
     for (int64_t i = a; i < b; ++i) sum += __ldcg(w.scnt + i);
-    uint32_t run = near_exsum<kNearThreads>(sum, wsum);
+    uint32_t run = near_exsum<NT>(sum, wsum);
     for (int64_t i = a; i < b; ++i) {
         w.soff[i] = run;
         run += __ldcg(w.scnt + i);
     }
-    if (threadIdx.x == kNearThreads - 1) {
+    if (threadIdx.x == NT - 1) {
         w.soff[nt] = run;
         w.ctl[2] = (int32_t)run;
         if (run <= (uint32_t)kNearCap) {
@@ -485,25 +508,39 @@ __device__ __forceinline__ int lower_bound_pairs(const uint64_t *sk, const uint3
     return lo;
 }
 
-__global__ void __launch_bounds__(kNearThreads) k_near_take(const uint64_t *__restrict__ keys,
+template <int NT>
+__global__ void __launch_bounds__(kNearTakeThreads) k_near_take(const uint64_t *__restrict__ keys,
                                                             int64_t nt, NearWs w) {
     __shared__ uint64_t sk[kNearCap];
     __shared__ uint32_t sp[kNearCap];
-    __shared__ uint32_t wsum[kNearThreads / 32];
     __shared__ int s_last;
     if (!ld_flag(w.ctl + 1)) return;
-    const int64_t t = blockIdx.x;
-    const uint32_t off0 = w.soff[t];
-    if (w.soff[t + 1] != off0) {
-        const int64_t base = t * kNearTile;
-        const int j0 = threadIdx.x * kNearItems;
-        const uint32_t sb = my_byte(w.bits + t * kNearWords);
-        uint32_t idx = off0 + near_exsum<kNearThreads>((uint32_t)__popc(sb), wsum);
+    // a warp per tile, the tile's bit words a few per lane
+    constexpr int kLaneWords = NearTile<NT>::words / 32;
+    const int lane = threadIdx.x & 31;
+    const int64_t t = blockIdx.x * (int64_t)kNearTakeTiles + (threadIdx.x >> 5);
+    const uint32_t off0 = t < nt ? w.soff[t] : 0u;
+    if (t < nt && w.soff[t + 1] != off0) {
+        uint32_t word[kLaneWords], cnt = 0;
 #pragma unroll
-        for (int q = 0; q < kNearItems; ++q) {
-            if ((sb >> q) & 1u) {
-                w.s_key[idx] = __ldg(keys + base + j0 + q);
-                w.s_pos[idx] = (uint32_t)(base + j0 + q);
+        for (int q = 0; q < kLaneWords; ++q) {
+            word[q] = w.bits[t * NearTile<NT>::words + lane * kLaneWords + q];
+            cnt += (uint32_t)__popc(word[q]);
+        }
+        uint32_t idx = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, idx, o);
+            if (lane >= o) idx += v;
+        }
+        idx += off0 - cnt;
+#pragma unroll
+        for (int q = 0; q < kLaneWords; ++q) {
+            const int64_t base = t * NearTile<NT>::keys + (lane * kLaneWords + q) * 32;
+            for (uint32_t left = word[q]; left; left &= left - 1u) {
+                const int64_t p = base + __ffs((int)left) - 1;
+                w.s_key[idx] = __ldg(keys + p);
+                w.s_pos[idx] = (uint32_t)p;
                 ++idx;
             }
         }
@@ -513,14 +550,14 @@ __global__ void __launch_bounds__(kNearThreads) k_near_take(const uint64_t *__re
     const int m = w.ctl[2];
     int P = 1;
     while (P < m) P <<= 1;
-    for (int i = threadIdx.x; i < P; i += kNearThreads) {
+    for (int i = threadIdx.x; i < P; i += kNearTakeThreads) {
         sk[i] = i < m ? __ldcg(w.s_key + i) : ~0ull;
         sp[i] = i < m ? __ldcg(w.s_pos + i) : kNone;
     }
     __syncthreads();
     for (int k = 2; k <= P; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P; i += kNearThreads) {
+            for (int i = threadIdx.x; i < P; i += kNearTakeThreads) {
                 const int ixj = i ^ j;
                 if (ixj > i) {
                     const bool up = (i & k) == 0;
@@ -534,16 +571,21 @@ __global__ void __launch_bounds__(kNearThreads) k_near_take(const uint64_t *__re
                     }
                 }
             }
-            __syncthreads();
+            // a distance below 32 stays within the elements of one warp
+            if (j >= 32 || (j == 1 && k >= 32))
+                __syncthreads();
+            else
+                __syncwarp();
         }
     }
-    for (int i = threadIdx.x; i < m; i += kNearThreads) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += kNearTakeThreads) {
         w.ss_key[i] = sk[i];
         w.ss_pos[i] = sp[i];
     }
     // per tile the S keys it places: from the first R key of the tile (tile 0:
     // from the start) to the first R key of a later tile (or the end)
-    for (int64_t u = threadIdx.x; u <= nt; u += kNearThreads) {
+    for (int64_t u = threadIdx.x; u <= nt; u += kNearTakeThreads) {
         int v;
         if (u == 0) {
             v = 0;
@@ -556,19 +598,20 @@ __global__ void __launch_bounds__(kNearThreads) k_near_take(const uint64_t *__re
     }
 }
 
-__global__ void __launch_bounds__(kNearThreads) k_near_place(const uint64_t *__restrict__ keys,
+template <int NT>
+__global__ void __launch_bounds__(NT) k_near_place(const uint64_t *__restrict__ keys,
                                                              int64_t n, NearWs w,
                                                              uint64_t *__restrict__ keys_out,
                                                              uint32_t *__restrict__ perm_out,
                                                              int32_t *flags, int64_t dest_bias) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t *rk = reinterpret_cast<uint64_t *>(smem);
-    uint32_t *rp = reinterpret_cast<uint32_t *>(smem + kNearTile * sizeof(uint64_t));
-    __shared__ uint32_t wsum[kNearThreads / 32];
+    uint32_t *rp = reinterpret_cast<uint32_t *>(smem + NearTile<NT>::keys * sizeof(uint64_t));
+    __shared__ uint32_t wsum[NT / 32];
     if (!ld_flag(w.ctl + 1)) return;
     const int64_t t = blockIdx.x;
-    const int64_t base = t * kNearTile;
-    const int own_n = (int)(n - base < kNearTile ? n - base : kNearTile);
+    const int64_t base = t * NearTile<NT>::keys;
+    const int own_n = (int)(n - base < NearTile<NT>::keys ? n - base : NearTile<NT>::keys);
     const int lo = (int)w.tlo[t], hi = (int)w.tlo[t + 1];
     const uint32_t soff = w.soff[t];
     const int s_tile = (int)(w.soff[t + 1] - soff);
@@ -595,12 +638,12 @@ __global__ void __launch_bounds__(kNearThreads) k_near_place(const uint64_t *__r
         return;
     }
     const int j0 = threadIdx.x * kNearItems;
-    const uint32_t sb = my_byte(w.bits + t * kNearWords);
+    const uint32_t sb = my_byte(w.bits + t * NearTile<NT>::words);
     uint64_t k[kNearItems];
 #pragma unroll
     for (int q = 0; q < kNearItems; ++q)
         k[q] = (j0 + q < own_n) ? __ldg(keys + base + j0 + q) : 0ull;
-    const uint32_t s_before = near_exsum<kNearThreads>((uint32_t)__popc(sb), wsum);
+    const uint32_t s_before = near_exsum<NT>((uint32_t)__popc(sb), wsum);
     // R keys of this tile, compacted in order
     uint32_t r_local = (uint32_t)j0 - s_before;
 #pragma unroll
@@ -634,7 +677,7 @@ __global__ void __launch_bounds__(kNearThreads) k_near_place(const uint64_t *__r
         }
     }
     const int r_tile = own_n - s_tile;
-    for (int s = lo + threadIdx.x; s < hi; s += kNearThreads) {
+    for (int s = lo + threadIdx.x; s < hi; s += NT) {
         const uint64_t ks = w.ss_key[s];
         const uint32_t ps = w.ss_pos[s];
         const int a = lower_bound_pairs(rk, rp, 0, r_tile, ks, ps);
@@ -651,8 +694,30 @@ __global__ void __launch_bounds__(kNearThreads) k_near_place(const uint64_t *__r
 }  // namespace
 
 int64_t near_bytes(int64_t n_max) {
-    const int64_t nt = (n_max + kNearTile - 1) / kNearTile;
+    constexpr int tile = NearTile<kNearMinThreads>::keys;
+    const int64_t nt = (n_max + tile - 1) / tile;
     return near_layout(nullptr, nt < 1 ? 1 : nt, nullptr);
+}
+
+template <int NT>
+static int launch_near(cnb_ctx *ctx, const NearWs &w, const uint64_t *keys_in, uint64_t *keys_out,
+                       uint32_t *perm_out, int64_t n, cudaStream_t st,
+                       cudaGraphConditionalHandle cond, bool use_cond) {
+    using T = NearTile<NT>;
+    const int64_t nt = (n + T::keys - 1) / T::keys;
+    CNB_CUDA(cudaFuncSetAttribute(k_near_mark<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)T::mark_smem));
+    CNB_CUDA(cudaFuncSetAttribute(k_near_place<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)T::place_smem));
+    k_near_mark<NT><<<(unsigned)nt, NT, T::mark_smem, st>>>(keys_in, n, nt, w);
+    CNB_TRY(launch_status());
+    k_near_filter<NT><<<(unsigned)nt, NT, 0, st>>>(keys_in, n, nt, w, ctx->sort_stats, cond, use_cond);
+    CNB_TRY(launch_status());
+    k_near_take<NT><<<(unsigned)((nt + kNearTakeTiles - 1) / kNearTakeTiles), kNearTakeThreads, 0, st>>>(keys_in, nt, w);
+    CNB_TRY(launch_status());
+    k_near_place<NT><<<(unsigned)nt, NT, T::place_smem, st>>>(keys_in, n, w, keys_out, perm_out,
+                                                              ctx->flags, ctx->near_dest_bias);
+    return launch_status();
 }
 
 // Launches the near-sorted path; *skip_full receives the device flag that
@@ -664,26 +729,22 @@ int sort_pairs_near(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
                     uint32_t *perm_out, int64_t n, cudaStream_t st, const int32_t **skip_full,
                     const int32_t **never, uint32_t **arrivals, cudaGraphConditionalHandle cond,
                     bool use_cond) {
-    const int64_t nt = (n + kNearTile - 1) / kNearTile;
-    const int64_t nt_max = (ctx->n_max + kNearTile - 1) / kNearTile;
+    constexpr int tile = NearTile<kNearMinThreads>::keys;
+    const int64_t nt_max = (ctx->n_max + tile - 1) / tile;
     NearWs w;
     near_layout(ctx->near, nt_max < 1 ? 1 : nt_max, &w);
     CNB_CUDA(cudaMemsetAsync(w.ctl, 0, 8 * sizeof(int32_t), st));
-    CNB_CUDA(cudaFuncSetAttribute(k_near_mark, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kNearMarkSmem));
-    CNB_CUDA(cudaFuncSetAttribute(k_near_place, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kNearPlaceSmem));
-    k_near_mark<<<(unsigned)nt, kNearThreads, kNearMarkSmem, st>>>(keys_in, n, nt, w);
-    CNB_TRY(launch_status());
-    k_near_filter<<<(unsigned)nt, kNearThreads, 0, st>>>(keys_in, n, nt, w, ctx->sort_stats, cond,
-                                                          use_cond);
-    CNB_TRY(launch_status());
-    k_near_take<<<(unsigned)nt, kNearThreads, 0, st>>>(keys_in, nt, w);
-    CNB_TRY(launch_status());
-    k_near_place<<<(unsigned)nt, kNearThreads, kNearPlaceSmem, st>>>(keys_in, n, w, keys_out,
-                                                                      perm_out, ctx->flags,
-                                                                      ctx->near_dest_bias);
-    CNB_TRY(launch_status());
+    // Small inputs leave the chip idle: more and smaller tiles shorten each one's chain of
+    // scans; large ones pay for every block's arrival at the counters (8 ns each on one address).
+    // Measured (us, the four kernels at 128 / 256 / 512 threads): 4 096 keys 15.2 / 15.6 / 16.8,
+    // 32 768 30.5 / 33.2 / 39.2, 100 003 33.0 / 35.7 / 42.2, 300 007 41.9 / 40.7 / 48.0, 1 000 003
+    // 60.6 / 60.8 / 63.7, 2 097 152 clustered 88.0 / 77.3 / 91.2, 8 000 000 163 / 108 / 86.
+    if (n <= 1 << 17)
+        CNB_TRY(launch_near<128>(ctx, w, keys_in, keys_out, perm_out, n, st, cond, use_cond));
+    else if (n <= 1 << 22)
+        CNB_TRY(launch_near<256>(ctx, w, keys_in, keys_out, perm_out, n, st, cond, use_cond));
+    else
+        CNB_TRY(launch_near<512>(ctx, w, keys_in, keys_out, perm_out, n, st, cond, use_cond));
     *skip_full = w.ctl + 1;
     *never = w.ctl + 7;  // zeroed with the rest of ctl, never set
     *arrivals = reinterpret_cast<uint32_t *>(w.ctl + 6);  // zeroed too

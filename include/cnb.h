@@ -112,7 +112,7 @@ int cnb_ctx_inject_sort_faults(cnb_ctx *ctx, int32_t wait_limit, int64_t withhel
  * CNB_SORT_FULL).  CNB_SORT_ADAPTIVE: cnb_sort_pairs with idx_in == NULL and
  * keys_in != keys_out first tries the near-sorted path -- keys that break
  * the ascending order (at every descent the shorter of the out-of-order runs
- * on its two sides, repeated in 4096-key windows until what is left ascends)
+ * on its two sides, repeated tile by tile until what is left ascends)
  * and keys outside the running max / min of the rest are taken out, sorted,
  * and merged back -- and runs the
  * full radix sort only when more than CNB_SORT_NEAR_CAP keys had to be
