@@ -137,7 +137,7 @@ __device__ __forceinline__ void apply_masked(const float4 *list, const uint2 *ma
         const float2 s2 = dup2(soft2);
         float2 fx = make_float2(ax[0], ax[1]), fy = make_float2(ay[0], ay[1]),
                fz = make_float2(az[0], az[1]);
-        // eight entries at a time: loads, distances and masses first, then the
+        // four entries at a time: loads, distances and masses first, then the
         // inverse cubes and the accumulation in list order
         int j = 0;
         for (; j + 4 <= cnt; j += 4) {
@@ -792,9 +792,10 @@ static int g_test_spill_every = 0;  // cnb_exact_test_spill
 
 // Systems of at most this many bodies take the walk by groups (forces_ref.cu):
 // their few hundred buckets leave most warps of the chip idle while each is a
-// serial walk of some 90 000 instructions.  Measured, theta 0.5 (us, buckets
-// against groups): 4 096 bodies 172 / 36, 32 768 412 / 141, 65 536 482 / 276,
-// 131 072 495 / 529.
+// serial walk of some 80 000 instructions.  Measured, theta 0.5, an even and a
+// clustered state (us, the faster bucket form against groups): 20 000 bodies
+// 160 and 208 / 87 and 95, 65 536 247 and 322 / 253 and 263, 98 000 312 and 396 /
+// 333 and 396, 131 072 364 and 510 / 470 and 533.
 constexpr int64_t kWalkBodies = 98304;
 
 int launch_exact(GroupedParams &P, int bodies_per_lane, int block_warps, cudaStream_t st) {

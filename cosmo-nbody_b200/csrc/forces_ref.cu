@@ -383,13 +383,14 @@ static int forces_walk(const float *px, const float *py, const float *pz, const 
     };
     // A smaller group shares less (more node fetches and tests in all) but gives more warps, and
     // below a few thousand warps a pass lasts as long as one warp's chain of fetches.  Measured
-    // (us, groups of 2 / 4 / 8 / 32): float32 4 096 targets 43 / 47 / 63 / 98, 32 768 93 / 76 / 75 /
-    // 98, 300 007 1585 / 1143 / 1033 / 1015, 2 097 152 12673 / 8820 / 7632 / 6775; float64 16 384
-    // 86 / 77 / 95 / 280, 300 007 1976 / 1640 / 1563 / 1823, 2 097 152 15709 / 12655 / 11504 / 11350
-    // (a test costs more there, so wasted lanes weigh more); EXACT 12 000 78 / 72 / 97 / 251,
-    // 65 536 326 / 276 / 286 / 399.
-    if (count <= 8192) return go(std::integral_constant<int, 2>());
-    if (EXACT || count <= 24576) return go(std::integral_constant<int, 4>());
+    // (us, groups of 2 / 4 / 8): float32 8 192 targets 51 / 55 / 71, 12 000 76 / 67 / 81, 24 576
+    // 129 / 112 / 109, 131 072 635 / 464 / 424; float64 (a test costs more there, so wasted lanes
+    // weigh more) 12 000 90 / 92 / 120, 48 000 291 / 261 / 293, 65 536 405 / 356 / 369, 131 072
+    // 801 / 675 / 671; EXACT 10 000 55 / 57 / 81, 12 000 69 / 62 / 87, 32 768 146 / 126 / 129, 65 536
+    // 304 / 251 / 256, 98 000 409 / 331 / 329.  Groups of 8 / 32: float32 300 007 1033 / 1015,
+    // 2 097 152 7632 / 6775; float64 300 007 1563 / 1823, 2 097 152 11504 / 11350.
+    if (count <= 10240) return go(std::integral_constant<int, 2>());
+    if (EXACT || count <= (sizeof(T) == 8 ? 65536 : 24576)) return go(std::integral_constant<int, 4>());
     if constexpr (!EXACT) {
         if (count <= (sizeof(T) == 8 ? 1 << 20 : 1 << 18)) return go(std::integral_constant<int, 8>());
         return go(std::integral_constant<int, 32>());
