@@ -32,6 +32,7 @@ constexpr int kIn = 12, kH = 64;
 constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kH * kIn, kOffW2 = kOffB1 + kH,
               kOffB2 = kOffW2 + kH * kH, kOffW3 = kOffB2 + kH, kOffB3 = kOffW3 + kH;
 constexpr int kParams = kOffB3 + 1;  // 5057
+constexpr int kMeanBodies = 64;  // largest bucket whose mean |a| a warp forms together
 constexpr float kThetaLo = 0.2f, kThetaHi = 1.0f;
 static_assert(kParams == CNB_MLP_PARAMS, "parameter count");
 
@@ -43,6 +44,11 @@ __device__ __forceinline__ float node_extent(const float4 *aabb, int v) {
     return fmaxf(hi.x - lo.x, fmaxf(hi.y - lo.y, hi.z - lo.z));
 }
 
+__device__ __forceinline__ float accel_norm(const float *__restrict__ accel, int64_t r) {
+    const float ax = accel[3 * r], ay = accel[3 * r + 1], az = accel[3 * r + 2];
+    return sqrtf(ax * ax + ay * ay + az * az);
+}
+
 // Mean |a| of a bucket's bodies (previous step; row perm[i] of accel for
 // sorted body i), by one thread.
 __device__ float bucket_mean_accel(const float *__restrict__ accel, const uint32_t *__restrict__ perm,
@@ -51,10 +57,64 @@ __device__ float bucket_mean_accel(const float *__restrict__ accel, const uint32
     for (int k = 0; k < bk.y; ++k) {
         const int64_t i = (int64_t)bk.x + k;
         const int64_t r = perm ? (int64_t)perm[i] : i;
-        const float ax = accel[3 * r], ay = accel[3 * r + 1], az = accel[3 * r + 2];
-        amean += sqrtf(ax * ax + ay * ay + az * az);
+        amean += accel_norm(accel, r);
     }
     return amean / (float)bk.y;
+}
+
+// The same means for a warp's 32 buckets, one per lane: the lanes fetch a
+// bucket's bodies together (their rows are nearly consecutive) into `row`,
+// half of the buckets at a time, and each lane adds up its own bucket in the
+// order above.  One thread per bucket alone waits for some fifty pairs of
+// dependent, uncoalesced loads: k_controller_mma on 42 000 buckets 105 us that
+// way, 61 together without the batches, 45 / 42 / 45 with batches of 2 / 4 / 8.
+// The rest of that kernel is 25 us: three levels of parents, one after the
+// other, and the network.
+constexpr int kMeanBatch = 4;
+static_assert(kMeanBodies == 64, "two rows a lane");
+constexpr int kMeanRow = kMeanBodies + 1;  // floats: staggers the banks
+__device__ __forceinline__ float warp_mean_accel(const float *__restrict__ accel,
+                                                 const uint32_t *__restrict__ perm, int4 bk, bool mine,
+                                                 float *row) {
+    const int lane = threadIdx.x & 31;
+    const bool staged = mine && bk.y <= kMeanBodies;
+    float amean = 0.f;
+    for (int half = 0; half < 32; half += 16) {
+        // kMeanBatch buckets at a time, every row's load in flight before the first is used
+        for (int b0 = 0; b0 < 16; b0 += kMeanBatch) {
+            int64_t r[kMeanBatch][2];
+            float norm[kMeanBatch][2];
+            bool ok[kMeanBatch][2];
+#pragma unroll
+            for (int u = 0; u < kMeanBatch; ++u) {
+                const int start = __shfl_sync(0xffffffffu, bk.x, half + b0 + u);
+                const int count = __shfl_sync(0xffffffffu, staged ? bk.y : 0, half + b0 + u);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = lane + 32 * h;
+                    ok[u][h] = k < count;
+                    const int64_t i = ok[u][h] ? (int64_t)start + k : 0;
+                    r[u][h] = perm ? (int64_t)__ldg(perm + i) : i;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kMeanBatch; ++u)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) norm[u][h] = accel_norm(accel, r[u][h]);
+#pragma unroll
+            for (int u = 0; u < kMeanBatch; ++u)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (ok[u][h]) row[(b0 + u) * kMeanRow + lane + 32 * h] = norm[u][h];
+        }
+        __syncwarp();
+        if (staged && (lane & 16) == half) {
+            for (int k = 0; k < bk.y; ++k) amean += row[(lane & 15) * kMeanRow + k];
+            amean /= (float)bk.y;
+        }
+        __syncwarp();
+    }
+    return mine && !staged ? bucket_mean_accel(accel, perm, bk) : amean;
 }
 
 __device__ void bucket_features(const float4 *__restrict__ rec, const float4 *__restrict__ aabb,
@@ -160,17 +220,21 @@ __global__ void __launch_bounds__(kMmaWarps * 32) k_controller_mma(
     const float *__restrict__ accel, const uint32_t *__restrict__ perm,
     const __nv_bfloat16 *__restrict__ wbf, float *__restrict__ theta, int max_buckets) {
     // float32: W1, b1, b2, w3, b3; bfloat16: W2 rows (output unit) of kHPad
-    __shared__ float w1[kH * kIn], b1[kH], b2[kH], w3[kH];
+    __shared__ __align__(16) float w1[kH * kIn];
+    __shared__ float b1[kH], b2[kH], w3[kH];
     __shared__ float b3;
     __shared__ __align__(16) __nv_bfloat16 w2[kH * kHPad];
     __shared__ __align__(16) __nv_bfloat16 hid[kMmaWarps][32 * kHPad];
-    for (int i = threadIdx.x; i < kH * kIn; i += blockDim.x) w1[i] = __bfloat162float(wbf[kOffW1 + i]);
-    for (int i = threadIdx.x; i < kH; i += blockDim.x) {
-        b1[i] = __bfloat162float(wbf[kOffB1 + i]);
-        b2[i] = __bfloat162float(wbf[kOffB2 + i]);
-        w3[i] = __bfloat162float(wbf[kOffW3 + i]);
+    constexpr int kThreads = kMmaWarps * 32;
+#pragma unroll
+    for (int i = threadIdx.x; i < kH * kIn; i += kThreads) w1[i] = __bfloat162float(wbf[kOffW1 + i]);
+    if (threadIdx.x < kH) {
+        b1[threadIdx.x] = __bfloat162float(wbf[kOffB1 + threadIdx.x]);
+        b2[threadIdx.x] = __bfloat162float(wbf[kOffB2 + threadIdx.x]);
+        w3[threadIdx.x] = __bfloat162float(wbf[kOffW3 + threadIdx.x]);
     }
-    for (int i = threadIdx.x; i < kH * kH; i += blockDim.x) w2[(i / kH) * kHPad + i % kH] = wbf[kOffW2 + i];
+#pragma unroll 16
+    for (int i = threadIdx.x; i < kH * kH; i += kThreads) w2[(i / kH) * kHPad + i % kH] = wbf[kOffW2 + i];
     if (threadIdx.x == 0) b3 = __bfloat162float(wbf[kOffB3]);
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -178,13 +242,15 @@ __global__ void __launch_bounds__(kMmaWarps * 32) k_controller_mma(
     const int nb = min(ws[0], max_buckets);
     const int4 *buckets = reinterpret_cast<const int4 *>(ws + 4);
     __nv_bfloat16 *h = hid[wib];
+    static_assert(sizeof(hid[0]) >= 16 * kMeanRow * sizeof(float), "the rows of warp_mean_accel");
     for (int base = (blockIdx.x * kMmaWarps + wib) * 32; base < nb; base += gridDim.x * kMmaWarps * 32) {
         // one bucket per lane: features and the first layer in float32
         const int g = base + lane;
+        const int4 bk = g < nb ? buckets[g] : make_int4(0, 0, 0, 0);
+        const float amean = warp_mean_accel(accel, perm, bk, g < nb, reinterpret_cast<float *>(h));
         if (g < nb) {
-            const int4 bk = buckets[g];
             float f[kIn];
-            bucket_features(rec, aabb, parents, bucket_mean_accel(accel, perm, bk), bk, f);
+            bucket_features(rec, aabb, parents, amean, bk, f);
 #pragma unroll 4
             for (int j = 0; j < kH; j += 2) {
                 float a0 = b1[j], a1 = b1[j + 1];

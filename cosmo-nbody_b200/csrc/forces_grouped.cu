@@ -51,6 +51,8 @@
 // Two bodies per lane run the force loop on packed float2 (FADD2 / FMUL2 /
 // FFMA2); the two-level walk (k_super_lists, cnb_forces_two_level) lets a
 // super-bucket walk the top of the tree once for all its buckets.
+#include <cooperative_groups.h>
+
 #include "grouped.cuh"
 
 namespace cnb {
@@ -807,32 +809,85 @@ __global__ void __launch_bounds__(256) k_pack_nodes(const float *__restrict__ n_
 
 // Heaviest buckets first: a counting sort of the bucket slots by theta in
 // 32 bins over [0.2, 1.0] (smallest theta = most interactions first), so the
-// persistent traversal does not end on a few expensive buckets.  One block;
-// the order inside a bin is whatever the atomics give (each bucket's result
-// does not depend on when it runs).
-constexpr int kOrderBins = 32;
-__global__ void __launch_bounds__(1024) k_order_buckets(const float *__restrict__ theta,
-                                                        const int32_t *__restrict__ ws,
-                                                        int32_t *__restrict__ order) {
-    __shared__ int32_t cnt[kOrderBins], start[kOrderBins];
+// persistent traversal does not end on a few expensive buckets.  One cluster
+// of eight blocks; a warp counts and places a contiguous part of the slots in
+// counters of its own, so no atomic is needed and slots keep their order inside
+// a bin.  Equal bins of 32 slots are found by one match.  Bound by one SM's
+// issue slots (eight SMs here): 42 000 slots 34 us with atomics on 32 addresses
+// in one block, 17 in one block this way, 6.4 in eight.
+constexpr int kOrderBins = 32, kOrderWarps = 32, kOrderBlocks = 8;
+__global__ void __cluster_dims__(kOrderBlocks, 1, 1) __launch_bounds__(kOrderWarps * 32)
+    k_order_buckets(const float *__restrict__ theta, const int32_t *__restrict__ ws,
+                    int32_t *__restrict__ order) {
+    namespace cg = cooperative_groups;
+    __shared__ int32_t at[kOrderWarps][kOrderBins];
+    __shared__ int32_t total[kOrderBins], before[kOrderBins];
+    cg::cluster_group cluster = cg::this_cluster();
     const int nb = ws[0];
-    if (threadIdx.x < kOrderBins) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    auto bin_of = [](float t) {
-        const int b = (int)((t - 0.2f) * (kOrderBins / 0.8f));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)cluster.block_rank();
+    constexpr int kAll = kOrderWarps * kOrderBlocks;
+    const int per = ((nb + kAll - 1) / kAll + 31) & ~31;
+    const int first = min((rank * kOrderWarps + warp) * per, nb), last = min(first + per, nb);
+    at[warp][lane] = 0;
+    __syncwarp();
+    const auto bin_of = [&](int g) {
+        if (g >= last) return kOrderBins;
+        const int b = (int)((theta[g] - 0.2f) * (kOrderBins / 0.8f));
         return b < 0 ? 0 : (b >= kOrderBins ? kOrderBins - 1 : b);
     };
-    for (int g = threadIdx.x; g < nb; g += blockDim.x) atomicAdd(&cnt[bin_of(theta[g])], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int b = 0; b < kOrderBins; ++b) {
-            start[b] = run;
-            run += cnt[b];
+    // the slots of this warp, 32 at a time; PLACE: at their bin's counter
+    const auto pass = [&](bool place) {
+        for (int base = first; base < last; base += 32 * 4) {
+            int bin[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) bin[u] = bin_of(base + u * 32 + lane);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t same = __match_any_sync(0xffffffffu, bin[u]);
+                const int nth = __popc(same & ((1u << lane) - 1u));
+                int pos = 0;
+                if (bin[u] < kOrderBins) {
+                    pos = at[warp][bin[u]] + nth;
+                    if (place) order[pos] = base + u * 32 + lane;
+                }
+                __syncwarp();
+                if (bin[u] < kOrderBins && (same >> lane) == 1u) at[warp][bin[u]] = pos + 1;
+                __syncwarp();
+            }
         }
-    }
+    };
+    pass(false);
     __syncthreads();
-    for (int g = threadIdx.x; g < nb; g += blockDim.x) order[atomicAdd(&start[bin_of(theta[g])], 1)] = g;
+    // counts to positions: by bin, then by block, then by warp; warp w scans bin w over the warps
+    static_assert(kOrderBins == 32 && kOrderWarps == 32, "a lane per warp, a warp per bin");
+    const int count = at[lane][warp];
+    int incl = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) total[warp] = incl;
+    cluster.sync();
+    if (warp == 0) {
+        int all = 0, lower = 0;  // of bin `lane`: over the cluster, over the blocks before this one
+        for (int r = 0; r < kOrderBlocks; ++r) {
+            const int t = *cluster.map_shared_rank(&total[lane], r);
+            all += t;
+            if (r < rank) lower += t;
+        }
+        int upto = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += t;
+        }
+        before[lane] = upto - all + lower;
+    }
+    cluster.sync();  // also: no block leaves while another reads its counts
+    at[lane][warp] = before[warp] + incl - count;
+    __syncthreads();
+    pass(true);
 }
 
 }  // namespace cnb
@@ -842,7 +897,7 @@ using namespace cnb;
 extern "C" int cnb_order_buckets(const float *theta_per_bucket, const int32_t *workspace,
                                  int32_t *order, void *stream) {
     if (!theta_per_bucket || !workspace || !order) return CNB_E_INVALID_ARG;
-    k_order_buckets<<<1, 1024, 0, as_stream(stream)>>>(theta_per_bucket, workspace, order);
+    k_order_buckets<<<kOrderBlocks, kOrderWarps * 32, 0, as_stream(stream)>>>(theta_per_bucket, workspace, order);
     return launch_status();
 }
 
