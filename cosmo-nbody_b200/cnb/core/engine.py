@@ -298,8 +298,10 @@ class SimulationEngine:
         self.a += 2 * self.da
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
+        launches = _lib.launch_count()
         with torch.cuda.graph(g):
             two_steps()
+        self.graph_launches = _lib.launch_count() - launches  # kernels in the graph's two steps
         self._graph = g
         self._graph_step = step0 + 2
         return g

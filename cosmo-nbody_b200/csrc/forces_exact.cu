@@ -66,7 +66,7 @@ namespace cnb {
 // walks those buckets again with a region of kXWordsRedo words, and drops what
 // does not fit there (CNB_FLAG_LIST_OVERFLOW).  Rounds are full until 480 of
 // the 640 words are used; the deepest use at theta = 0.5 on 128^3 and 256^3
-// Zel'dovich and evolved states (two-level walk included) is 585 words.
+// Zel'dovich and evolved states (two-level walk included) is 607 words.
 // 640 against 864 words (and 2048 at small angles or with several boxes, as
 // one size used to need): theta 0.3 500k bodies 4.72 -> 4.35 ms, 16 boxes
 // 1.48 -> 1.37; 512 and 496 are no faster.
