@@ -4,8 +4,9 @@
 //
 // A bucket is a maximal radix-tree subtree with at most 32*BPL bodies
 // (cnb_make_buckets), so it is contiguous in the sorted order and spatially
-// compact.  One warp takes a bucket (dynamic scheduling: an atomic work
-// counter), each lane holds BPL bodies.  The warp walks the tree 32 nodes at
+// compact.  One warp takes a bucket, or in small systems a team of the block's
+// warps (see team_warps), by dynamic scheduling (an atomic work counter); each
+// lane holds BPL bodies.  The warp walks the tree 32 nodes at
 // a time from a per-warp node stack in shared memory: each lane tests one
 // node against the bucket's bounding box, accepted nodes (and reached
 // leaves) are appended to a per-warp interaction list in shared memory with
@@ -130,11 +131,6 @@ template <int BPL, bool QUAD> __host__ __device__ constexpr int second_width() {
     return QUAD ? 3 : entry_width<BPL>();
 }
 
-// The exact minimum-image test (CNB_MAC_PERIODIC) opens every node whose
-// image box can reach a bucket and walks far wider than the other tests:
-// its node stack is this many entries per warp.
-constexpr int kGStackPeriodic = 4096;
-
 // the table points of the two lists' entries (quadrupole entries hold their own)
 template <int LAW> __host__ __device__ constexpr int cell_words() {
     return LAW == 0 ? 0 : LAW == 1 ? 2 * kGList : kGList;
@@ -238,16 +234,20 @@ struct EwaldSums {
 // LAW: 0 the minimum-image laws (CNB_MAC_REF_X, CNB_MAC_PERIODIC), 1 the
 // periodic (Ewald) law with monopoles, 2 the periodic law with quadrupoles.
 // Warps per SM the registers are bounded for, by measurement: law 0 24 (77 registers: 128^3 bucket
-// test 2.00 ms; 28 and 20: 2.02, 2.06), with the large stack 8 (128 registers: shared memory
-// keeps it at 11 warps anyway, 30k bodies 1.31 ms against 1.42 with 66 registers); law 1 28 (72
-// registers: 128^3 4.31 ms; left alone the compiler takes 64 and 4.48 ms), law 2 20 (95 registers:
-// 300k bodies 1.155 ms; 24: 1.23).
-template <int LAW, int STACK> __host__ __device__ constexpr int law_warps() {
-    return LAW == 1 ? 28 : LAW == 2 ? 20 : STACK > kGStack ? 8 : 24;
+// test 2.00 ms; 28 and 20: 2.02, 2.06); law 1 28 (72 registers: 128^3 4.31 ms; left alone the
+// compiler takes 64 and 4.48 ms), law 2 20 (95 registers: 300k bodies 1.155 ms; 24: 1.23).
+template <int LAW> __host__ __device__ constexpr int law_warps() {
+    return LAW == 1 ? 28 : LAW == 2 ? 20 : 24;
 }
 
-template <int BPL, int WARPS, int LAW, int STACK>
-__global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k_forces_grouped(GroupedParams P) {
+// TEAM: the block's warps walk a bucket together, from one stack of STACK
+// entries that they pop in turn: every warp classifies its share of a round's
+// nodes and applies what it accepts to all of the bucket's bodies from lists of
+// its own, and warp 0 adds the warps' sums up in their order.  A round pops at
+// most a fifth of the free entries (a popped one leaves one more at most), so a
+// walk that fills the stack narrows to a depth-first one.
+template <int BPL, int WARPS, int LAW, int STACK, bool TEAM = false>
+__global__ void __launch_bounds__(WARPS * 32, law_warps<LAW>() / WARPS) k_forces_grouped(GroupedParams P) {
     constexpr bool EWALD = LAW != 0;
     constexpr bool QUAD = LAW == 2;
     extern __shared__ __align__(16) unsigned char g_smem[];
@@ -262,8 +262,10 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
     float4 *wlist = list + kGList * EW;
     int32_t *stack =
         reinterpret_cast<int32_t *>(g_smem + WARPS * kGList * (EW + SW) * sizeof(float4)) +
-        wib * (STACK + cell_words<LAW>());
-    uint32_t *cells = reinterpret_cast<uint32_t *>(stack + STACK);
+        (TEAM ? 0 : wib * (STACK + cell_words<LAW>()));
+    uint32_t *cells = reinterpret_cast<uint32_t *>(stack + STACK) + (TEAM ? wib * cell_words<LAW>() : 0);
+    // TEAM: the bucket, and per warp the nodes it opened this round and its entries
+    __shared__ int s_bucket, s_open[TEAM ? WARPS : 1], s_entries[TEAM ? WARPS : 1];
     unsigned long long n_tests = 0;
     int max_top = 0;
     bool overflow = false;
@@ -272,8 +274,14 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
 
     for (;;) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(P.ws + 1, 1);
-        g = __shfl_sync(0xffffffffu, g, 0);
+        if (TEAM) {
+            if (threadIdx.x == 0) s_bucket = atomicAdd(P.ws + 1, 1);
+            __syncthreads();
+            g = s_bucket;
+        } else {
+            if (lane == 0) g = atomicAdd(P.ws + 1, 1);
+            g = __shfl_sync(0xffffffffu, g, 0);
+        }
         if (g >= n_buckets) break;
         if (P.bucket_order) g = P.bucket_order[g];
         const int4 bk = P.buckets[g];
@@ -339,24 +347,29 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
             if (h.w) {
                 // the far field the super-bucket accepted holds for this bucket too
                 const float4 *far = P.far_lists + (int64_t)sup * P.far_cap;
-                for (int j0 = 0; j0 < h.x; j0 += 32) {
+                constexpr int kStep = TEAM ? 32 * WARPS : 32;
+                const int first = TEAM ? 32 * wib : 0;
+                for (int j0 = first; j0 < h.x; j0 += kStep) {
                     const int c = min(32, h.x - j0);
                     if (lane < c) put_entry<BPL>(list, lane, far[j0 + lane]);
                     __syncwarp();
                     apply_entries<BPL, false, false>(list, c, x, y, z, soft2, ax, ay, az);
                     __syncwarp();
                 }
-                for (int j0 = 0; j0 < h.y; j0 += 32) {
+                for (int j0 = first; j0 < h.y; j0 += kStep) {
                     const int c = min(32, h.y - j0);
                     if (lane < c) put_entry<BPL>(list, lane, far[P.far_cap - h.y + j0 + lane]);
                     __syncwarp();
                     apply_entries<BPL, true, true>(list, c, x, y, z, soft2, ax, ay, az);
                     __syncwarp();
                 }
-                n_entries += h.x + h.y;
-                n_wrap += h.y;
+                if (!TEAM || wib == 0) {
+                    n_entries += h.x + h.y;
+                    n_wrap += h.y;
+                }
                 // the near nodes it left are this bucket's starting stack
                 const int32_t *near = P.near_lists + (int64_t)sup * P.near_cap;
+                // (TEAM: every warp writes all of it, the same values)
                 for (int j = lane; j < h.z; j += 32) stack[j] = near[j];
                 top = h.z;
                 seeded = true;
@@ -421,11 +434,23 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
                 if (lane == 0) set_flag(P.status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
-            const int k = top < 32 ? top : 32;
-            top -= k;
             int32_t node = -1;
-            if (lane < k) node = stack[top + lane];
-            __syncwarp();
+            if (TEAM) {
+                const int k = min(min(top, 32 * WARPS), (STACK - top + 4) / 5);
+                if (k <= 0) {
+                    overflow = true;  // nodes dropped (flagged)
+                    break;
+                }
+                top -= k;
+                __syncthreads();  // the last round's pushes
+                const int e = wib + WARPS * lane;
+                if (e < k) node = stack[top + e];
+            } else {
+                const int k = top < 32 ? top : 32;
+                top -= k;
+                if (lane < k) node = stack[top + lane];
+                __syncwarp();
+            }
             if (node >= P.m_nodes) {
                 set_flag(P.status, CNB_FLAG_BAD_TOPOLOGY);
                 node = -1;
@@ -522,8 +547,25 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
             }
             cnt += __popc(nm);
             wcnt += __popc(wm);
-            const int nopen = __popc(om);
-            if (top + 2 * nopen > STACK) {
+            int nopen = __popc(om);
+            if (TEAM) {
+                if (lane == 0) s_open[wib] = nopen;
+                __syncthreads();  // every warp has read its nodes
+                int before = 0;
+                nopen = 0;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) {
+                    if (w == wib) before = nopen;
+                    nopen += s_open[w];
+                }
+                if (open) {
+                    const int pos = top + 2 * (before + __popc(om & lt));
+                    stack[pos] = c1;
+                    stack[pos + 1] = c0;
+                }
+                top += 2 * nopen;
+                max_top = max(max_top, top);
+            } else if (top + 2 * nopen > STACK) {
                 overflow = true;  // children dropped (flagged)
             } else {
                 if (open) {
@@ -588,9 +630,36 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
                 az[b] += es.g[2] + es.j[2] * ux + es.j[4] * uy + es.j[5] * uz - lin * cz;
             }
         }
+        uint32_t bucket_entries = n_entries;
+        if (TEAM) {
+            // the warps' sums through their lists' memory, added by warp 0 in their order
+            constexpr int kStride = kGList * (EW + SW) * 4;  // floats of a warp's lists
+            float *sum = reinterpret_cast<float *>(list);
+#pragma unroll
+            for (int b = 0; b < BPL; ++b) {
+                sum[(3 * b) * 32 + lane] = ax[b];
+                sum[(3 * b + 1) * 32 + lane] = ay[b];
+                sum[(3 * b + 2) * 32 + lane] = az[b];
+            }
+            if (lane == 0) s_entries[wib] = (int)n_entries;
+            __syncthreads();
+            if (wib == 0) {
+                for (int w = 1; w < WARPS; ++w) {
+                    const float *other = sum + w * kStride;
+#pragma unroll
+                    for (int b = 0; b < BPL; ++b) {
+                        ax[b] += other[(3 * b) * 32 + lane];
+                        ay[b] += other[(3 * b + 1) * 32 + lane];
+                        az[b] += other[(3 * b + 2) * 32 + lane];
+                    }
+                    bucket_entries += (uint32_t)s_entries[w];
+                }
+            }
+        }
+        const bool writer = !TEAM || wib == 0;
 #pragma unroll
         for (int b = 0; b < BPL; ++b) {
-            if (valid[b]) {
+            if (valid[b] && writer) {
                 const int64_t i = (int64_t)bk.x + lane + 32 * b;
                 const float fx = P.G * ax[b], fy = P.G * ay[b], fz = P.G * az[b];
                 P.force[3 * i] = fx;
@@ -600,7 +669,7 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW, STACK>() / WARPS) k
                     set_flag(P.status, CNB_FLAG_NONFINITE);
             }
         }
-        if (P.bucket_inter && lane == 0) P.bucket_inter[g] = (int32_t)n_entries;
+        if (P.bucket_inter && lane == 0 && writer) P.bucket_inter[g] = (int32_t)bucket_entries;
         if (P.stats && lane == 0) {
             atomicAdd(P.stats, n_entries * (unsigned long long)count);
             atomicAdd(P.stats + 2, n_wrap * (unsigned long long)count);
@@ -917,8 +986,9 @@ extern "C" int cnb_pack_nodes(const float *n_mass, const float *n_com, const flo
     return launch_status();
 }
 
-template <int BPL, int WARPS, int LAW, int STACK>
+template <int BPL, int WARPS, int LAW>
 static int launch_shape(GroupedParams &P, cudaStream_t st) {
+    constexpr int STACK = kGStack;
     const size_t smem = grouped_smem<BPL, LAW>(WARPS, STACK);
     CNB_CUDA(cudaFuncSetAttribute(k_forces_grouped<BPL, WARPS, LAW, STACK>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -931,18 +1001,77 @@ static int launch_shape(GroupedParams &P, cudaStream_t st) {
     return launch_status();
 }
 
+template <int BPL, int WARPS, int LAW, int STACK>
+static int launch_team(GroupedParams &P, cudaStream_t st) {
+    constexpr size_t smem = grouped_smem<BPL, LAW>(WARPS, 0) + STACK * sizeof(int32_t);
+    const auto kernel = k_forces_grouped<BPL, WARPS, LAW, STACK, true>;
+    CNB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, WARPS * 32, smem);
+    kernel<<<kSMs * (per_sm > 0 ? per_sm : 1), WARPS * 32, smem, st>>>(P);
+    return launch_status();
+}
+
+// The stack of a team grows with the entries it pops a round; the minimum-image
+// test opens every node whose image box can reach a bucket, walks far wider
+// than the others and gets three times as much.
+template <int BPL, int WARPS>
+static int launch_team_law(GroupedParams &P, cudaStream_t st) {
+    constexpr int STACK = 512 + 256 * WARPS, STACK_PERIODIC = 512 + 768 * WARPS;
+    if (P.mac == CNB_MAC_PERIODIC) return launch_team<BPL, WARPS, 0, STACK_PERIODIC>(P, st);
+    if (P.mac != CNB_MAC_EWALD) return launch_team<BPL, WARPS, 0, STACK>(P, st);
+    return P.quad ? launch_team<BPL, WARPS, 2, STACK>(P, st) : launch_team<BPL, WARPS, 1, STACK>(P, st);
+}
+
+template <int BPL>
+static int launch_team_size(GroupedParams &P, int warps, cudaStream_t st) {
+    switch (warps) {
+        case 2: return launch_team_law<BPL, 2>(P, st);
+        case 4: return launch_team_law<BPL, 4>(P, st);
+        default: return launch_team_law<BPL, 8>(P, st);
+    }
+}
+
+// How many warps walk a bucket together.  A small system has fewer buckets than
+// the chip holds warps (3000 to 4000), and a pass lasts as long as one warp's chain of
+// node fetches and lists; a team shortens the chain and pays for it with two
+// barriers a round, lanes without a node and its lists' remainders, so it is
+// wanted while its blocks (444, 1036 or 2072 resident for the periodic law, less
+// with quadrupoles) take about all buckets at once.  The minimum-image test's
+// chains are so long, and its stack so large, that two warps are never worse.
+// Measured (us, 1 / 2 / 4 / 8 warps, 64-body buckets; the lines of 32-body ones
+// lie at about half the bodies): periodic law 4 096 bodies 104 / 93 / 68 / 47,
+// 24 576 176 / 146 / 97 / 87, 65 536 217 / 167 / 162 / 179, 131 072 292 / 307 / 310 / 371;
+// quadrupoles 12 288 161 / 112 / 82 / 56, 16 384 175 / 128 / 92 / 93, 65 536 172 / 140 /
+// 146 / 216, 100 003 225 / 226 / 248 / 364; bucket test 24 576 142 / 110 / 72 / 71, 50 000 184 /
+// 136 / 121 / 135, 114 688 224 / 220 / 235 / 288; minimum image 12 288 687 / 722 / 444 /
+// 270, 50 000 2170 / 2159 / 1601 / 1591, 200 003 14.4 / 11.0 / 11.3 / 12.3 ms.
+static int team_warps(const GroupedParams &P, int bodies_per_lane) {
+    const bool wide = bodies_per_lane == 2;
+    struct { int64_t eight, four, two; } most;  // bodies
+    if (P.mac == CNB_MAC_PERIODIC)
+        most = wide ? decltype(most){49152, 65536, INT64_MAX} : decltype(most){12288, 49152, INT64_MAX};
+    else if (P.mac != CNB_MAC_EWALD)
+        most = wide ? decltype(most){24576, 49152, 114688} : decltype(most){8192, 24576, 57344};
+    else if (P.quad)
+        most = wide ? decltype(most){12288, 49152, 98304} : decltype(most){6144, 20480, 32768};
+    else
+        most = wide ? decltype(most){24576, 65536, 98304} : decltype(most){8192, 32768, 40960};
+    return P.n <= most.eight ? 8 : P.n <= most.four ? 4 : P.n <= most.two ? 2 : 1;
+}
+
 template <int BPL, int WARPS>
 static int launch_law(GroupedParams &P, cudaStream_t st) {
-    if (P.mac == CNB_MAC_PERIODIC) return launch_shape<BPL, WARPS, 0, kGStackPeriodic>(P, st);
-    if (P.mac != CNB_MAC_EWALD) return launch_shape<BPL, WARPS, 0, kGStack>(P, st);
-    return P.quad ? launch_shape<BPL, WARPS, 2, kGStack>(P, st)
-                  : launch_shape<BPL, WARPS, 1, kGStack>(P, st);
+    if (P.mac != CNB_MAC_EWALD) return launch_shape<BPL, WARPS, 0>(P, st);
+    return P.quad ? launch_shape<BPL, WARPS, 2>(P, st) : launch_shape<BPL, WARPS, 1>(P, st);
 }
 
 static int launch_grouped(GroupedParams &P, int bodies_per_lane, int block_warps,
                           cudaStream_t st) {
     CNB_CUDA(cudaMemsetAsync(P.ws + 1, 0, 2 * sizeof(int32_t), st));
     if (P.mac == CNB_MAC_REF_X) return launch_exact(P, bodies_per_lane, block_warps, st);
+    const int team = team_warps(P, bodies_per_lane);
+    if (team > 1) return bodies_per_lane == 2 ? launch_team_size<2>(P, team, st) : launch_team_size<1>(P, team, st);
     switch (bodies_per_lane * 16 + block_warps) {
         case 16 + 2: return launch_law<1, 2>(P, st);
         case 16 + 4: return launch_law<1, 4>(P, st);
