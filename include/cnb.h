@@ -271,7 +271,8 @@ int cnb_build_tree_ranges(const uint64_t *codes, int32_t *children, int32_t *par
  * [2] deepest node stack seen by the traversal (entries; for CNB_MAC_REF_X
  * words of its stack region, one per whole-bucket entry and three per
  * part-bucket entry: 640 words in the main pass, 4096 when a bucket is walked
- * again; small systems, walked by groups of bodies: entries), [3] the bodies' (index + 1)
+ * again; small systems, walked by groups of bodies or by teams of warps whose
+ * size does not follow block_warps: entries of a group or team), [3] the bodies' (index + 1)
  * summed over all buckets modulo 2^32 (N(N+1)/2 when the buckets tile the
  * bodies once; cnb_upward_table_buckets flags CNB_FLAG_BAD_TOPOLOGY
  * otherwise, and also when a bucket's nodes do not form a tree over its
