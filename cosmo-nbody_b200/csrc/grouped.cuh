@@ -78,13 +78,12 @@ constexpr float kCutGuard = 2e-7f;
 constexpr float kBoxSlack = 1e-6f;
 constexpr float kRelMargin = 4e-6f;
 
-// 1 / sqrt(q) for q of at least kMinSoft2.  rsqrtf also serves subnormal q, at
-// three more instructions a call (a compare and two scalings); the force loops
-// raise eps^2 to the smallest normal float, which no pair beyond the cut
-// (d^2 > 1e-7) can see and which leaves q = d^2 + eps^2 normal for every pair.
-// A packed pair of interactions is 17 instructions instead of 23: bucket test
-// 128^3 2.30 -> 2.01 ms, exact test 4.74 -> 4.48, periodic law 4.75 -> 4.46,
-// float32 per-body walk 6.78 -> 6.22 ms.
+// 1 / sqrt(q) for q of at least kMinSoft2, by the flush-to-zero form of PTX's
+// approximate reciprocal square root, whose results are defined for normal q.
+// The force loops raise eps^2 to the smallest normal float, which no pair
+// beyond the cut (d^2 > 1e-7) can see and which leaves q = d^2 + eps^2 normal
+// for every pair.  Against rsqrtf: bucket test 128^3 2.30 -> 2.01 ms, exact test
+// 4.74 -> 4.48, periodic law 4.75 -> 4.46, float32 per-body walk 6.78 -> 6.22 ms.
 constexpr float kMinSoft2 = 1.17549435e-38f;
 __device__ __forceinline__ float rsqrt_normal(float q) {
     float r;
