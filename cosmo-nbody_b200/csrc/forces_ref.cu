@@ -148,9 +148,19 @@ __device__ __noinline__ void walk_one(const RefTree<T> &R, int32_t root, float x
 // thread per target against this, same values: float32 2 097 152 targets theta
 // 0.5 41.7 -> 6.8 ms, 32 768 with the reference's scattered keys 48.0 -> 3.9 ms;
 // float64 2 097 152 37.3 -> 11.4 ms, 5 000 of 64 000 840 -> 80 us.
+//
+// The stack never fills on a radix tree.  A popped entry leaves at most one more
+// than it took, so popping a quarter of what is free below kRefWide keeps rounds
+// of several entries within kRefWide; from there on a round pops one, and a
+// depth-first walk holds at most an entry a level more.  The levels of a tree
+// over 64-bit keys, runs of equal ones split by index, are at most 64 + 32: the
+// kRefStack - kRefWide entries kept for it are more.  Only a caller's own,
+// deeper tree can fill the stack.
 constexpr int kRefWarps = 4;
 constexpr int kRefStack = 512;   // entries of a warp's shared stack
+constexpr int kRefWide = kRefStack - 128;
 constexpr int kRefDepth = 63;
+static_assert(kRefStack - kRefWide > 64 + 32, "a level each for a depth-first walk");
 
 // What a step reads of an entry, two 128-bit words: (com, w) and
 //   float:  (G m, sx^2 or -1 for a leaf, targets, 0)
@@ -205,9 +215,8 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     }
     __syncwarp();
     while (top > 0) {
-        // fewer as the stack fills (a popped entry leaves at most one more than it took), so that
-        // a walk that opens everything narrows to a depth-first one
-        const int room = (kRefStack - top) >> 3;
+        // fewer as the stack fills, down to a depth-first walk
+        const int room = (kRefWide - top) >> 2;
         const int k = min(top, min(32, room > 1 ? room : 1));
         top -= k;
         popped += k;

@@ -1,0 +1,61 @@
+"""Small systems whose trees are as deep as the keys allow: a cusp around a
+corner of the box, every body in a key cell of its own, 64 levels.  Every node
+that a walk opens leaves a sibling behind on each level, so the traversals'
+stacks fill at the angles where they are widest; none may drop a node."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+SOFT = 1e-3
+
+
+def _cusp(n, seed):
+    rng = np.random.default_rng(seed)
+    p = np.abs(rng.normal(size=(2 * n, 3))) ** 3 * 2.0 ** (-16 * rng.random((2 * n, 1))) * 0.3
+    p = (p % 1.0).astype(np.float32)
+    p[p >= 1] = 0
+    codes, _ = orc.compute_codes(p[:, 0], p[:, 1], p[:, 2], 1)
+    first = np.sort(np.unique(codes, return_index=True)[1])[:n]
+    p, codes = p[first], codes[first]
+    assert codes.size == n
+    perm = orc.argsort_stable(codes)
+    return [np.ascontiguousarray(p[perm][:, k]) for k in range(3)], codes[perm]
+
+
+def _cuda(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+# groups of 2 and of 4 targets
+@pytest.mark.parametrize("n", [10240, 59145])
+@pytest.mark.parametrize("theta", [0.1, 0.2, 0.3])
+def test_exact_decisions_by_groups(n, theta):
+    """The accepted (body, node) pairs are the oracle's, count for count; float32
+    sums of at most n = 6e4 terms rounded to 2^-24: a random walk of sqrt(n)
+    roundings is 1.5e-5 of the summed magnitudes, which are at most a few
+    times the largest force in a cusp: 1e-4."""
+    from cnb import _lib
+    from cnb.core.octree import OctreeManager
+    pos, codes = _cusp(n, 1)
+    mass = np.full(n, 1.0 / n, np.float32)
+    ch, par = orc.build_tree(codes)
+    nm, nc, lo, hi = orc.compute_multipoles(*pos, mass, ch, par)
+    want, dropped, _, acc = orc.compute_forces(*pos, ch, nm, nc, lo, hi, theta, 1.0, SOFT, 1.0,
+                                               orc.find_root(par), return_accepted=True)
+    assert dropped == 0
+    P = [_cuda(a) for a in pos]
+    tm = OctreeManager(n, node_table=True, bucket=64)
+    tm.build(P, _cuda(mass), _cuda(codes))
+    f = torch.empty((n, 3), device="cuda")
+    stats = torch.zeros(4, dtype=torch.int64, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.call("cnb_forces_grouped", *(q.data_ptr() for q in P), tm.node_table.data_ptr(),
+              tm.workspace.data_ptr(), f.data_ptr(), n, theta, None, _lib.MAC_REF_X, 2, 4, 1.0, SOFT, 1.0,
+              0.0, stats.data_ptr(), status.data_ptr(), int(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert int(stats[0]) == acc
+    assert np.abs(f.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
