@@ -244,8 +244,11 @@ template <int LAW> __host__ __device__ constexpr int law_warps() {
 // entries that they pop in turn: every warp classifies its share of a round's
 // nodes and applies what it accepts to all of the bucket's bodies from lists of
 // its own, and warp 0 adds the warps' sums up in their order.  A round pops at
-// most a fifth of the free entries (a popped one leaves one more at most), so a
-// walk that fills the stack narrows to a depth-first one.
+// most a fifth of what is free below STACK - kTeamDeep (a popped entry leaves one
+// more at most), and one entry above: a depth-first walk, which holds at most an
+// entry a level more, and a radix tree over 64-bit keys has at most 64 + 32
+// levels.  Only a caller's own, deeper tree can fill the stack.
+constexpr int kTeamDeep = 128;
 template <int BPL, int WARPS, int LAW, int STACK, bool TEAM = false>
 __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW>() / WARPS) k_forces_grouped(GroupedParams P) {
     constexpr bool EWALD = LAW != 0;
@@ -436,8 +439,8 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW>() / WARPS) k_forces
             }
             int32_t node = -1;
             if (TEAM) {
-                const int k = min(min(top, 32 * WARPS), (STACK - top + 4) / 5);
-                if (k <= 0) {
+                const int k = min(min(top, 32 * WARPS), max((STACK - kTeamDeep - top + 4) / 5, 1));
+                if (top >= STACK) {
                     overflow = true;  // nodes dropped (flagged)
                     break;
                 }
@@ -1017,7 +1020,7 @@ static int launch_team(GroupedParams &P, cudaStream_t st) {
 // than the others and gets three times as much.
 template <int BPL, int WARPS>
 static int launch_team_law(GroupedParams &P, cudaStream_t st) {
-    constexpr int STACK = 512 + 256 * WARPS, STACK_PERIODIC = 512 + 768 * WARPS;
+    constexpr int STACK = 512 + 256 * WARPS + kTeamDeep, STACK_PERIODIC = 512 + 768 * WARPS + kTeamDeep;
     if (P.mac == CNB_MAC_PERIODIC) return launch_team<BPL, WARPS, 0, STACK_PERIODIC>(P, st);
     if (P.mac != CNB_MAC_EWALD) return launch_team<BPL, WARPS, 0, STACK>(P, st);
     return P.quad ? launch_team<BPL, WARPS, 2, STACK>(P, st) : launch_team<BPL, WARPS, 1, STACK>(P, st);

@@ -59,3 +59,44 @@ def test_exact_decisions_by_groups(n, theta):
     assert int(status.item()) == 0
     assert int(stats[0]) == acc
     assert np.abs(f.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
+
+
+# per law and bucket width a size for teams of eight, four and two warps
+TEAMS = {("bucket", 2): (20000, 40000, 70000), ("bucket", 1): (8000, 20000, 40000),
+         ("periodic", 2): (20000, 59145, 70000), ("periodic", 1): (12000, 40000, 59145),
+         ("ewald", 2): (20000, 59145, 70000), ("ewald", 1): (8000, 30000, 40000),
+         ("quad", 2): (12000, 40000, 70000), ("quad", 1): (6000, 20000, 30000)}
+
+
+@pytest.mark.parametrize("theta", [0.0, 0.1, 0.2])
+@pytest.mark.parametrize("law,bpl,n", [(law, bpl, n) for law, bpl in TEAMS for n in TEAMS[law, bpl]])
+def test_teams_drop_nothing(law, bpl, n, theta):
+    """No node is dropped (the status says so); at theta = 0 every body meets
+    every leaf exactly once."""
+    from cnb import _lib
+    from cnb.core.octree import OctreeManager
+    pos, codes = _cusp(n, 3)
+    P = [_cuda(a) for a in pos]
+    tm = OctreeManager(n, node_table=True, bucket=32 * bpl, quad=law == "quad")
+    tm.build(P, torch.full((n,), 1.0 / n, device="cuda"), _cuda(codes))
+    f = torch.full((n, 3), float("nan"), device="cuda")
+    stats = torch.zeros(4, dtype=torch.int64, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    st = int(torch.cuda.current_stream().cuda_stream)
+    head = [q.data_ptr() for q in P] + [tm.node_table.data_ptr(), tm.workspace.data_ptr(), f.data_ptr(), n,
+                                        theta, None]
+    if law in ("ewald", "quad"):
+        table = torch.empty((9 ** 3, 24), device="cuda")
+        _lib.call("cnb_ewald_table", table.data_ptr(), 8, st)
+        _lib.call("cnb_forces_grouped_ewald", *head, bpl, 4, 1.0, SOFT, table.data_ptr(), 8,
+                  tm.quad.data_ptr() if law == "quad" else None, None, None, stats.data_ptr(),
+                  status.data_ptr(), st)
+    else:
+        mac = _lib.MAC_PERIODIC if law == "periodic" else _lib.MAC_REF_X_BUCKET
+        _lib.call("cnb_forces_grouped", *head, mac, bpl, 4, 1.0, SOFT, 1.0, 0.0, stats.data_ptr(),
+                  status.data_ptr(), st)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert bool(torch.isfinite(f).all())
+    if theta == 0.0:
+        assert int(stats[0]) == n * n
