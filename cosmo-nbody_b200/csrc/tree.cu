@@ -369,14 +369,15 @@ template <bool COMP>
 __device__ __forceinline__ void climb_global(const NodeArrays &A, int64_t curr, int32_t p, Acc a,
                                              const int32_t *__restrict__ children,
                                              const int32_t *__restrict__ parents, int32_t *counts,
-                                             int64_t m_nodes, int32_t *status) {
+                                             int64_t n, int32_t *status) {
+    const int64_t m_nodes = 2 * n - 1;
     for (int64_t guard = 0;; ++guard) {
         if (guard > m_nodes) {
             set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
             return;
         }
         if (p == -1) return;
-        if (p < 0 || p >= m_nodes) {
+        if (p < n || p >= m_nodes) {  // a parent is an internal node
             set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
             return;
         }
@@ -409,9 +410,10 @@ __device__ __forceinline__ void climb_global(const NodeArrays &A, int64_t curr, 
 // consecutive addresses on consecutive threads, their counters set to the two
 // arrivals.  A node whose parent is outside the block, or whose parent saw no
 // second arrival in the block, is left for the second launch: the block lists
-// them in its part of the leaves' counters (otherwise unused and zero).
-// k_upward_rest climbs from the listed nodes with the global counters, and
-// zeroes the list.
+// them in its part of the leaves' counters, which have no other use; it writes
+// all of that part, whatever it held.  k_upward_rest climbs from the listed
+// nodes with the global counters, and zeroes the list.  A climb ends where a
+// parent is no internal node, so it never counts an arrival in the list.
 //
 // HBM-bound in principle (88 bytes a node: values out, topology in).  One
 // climb per leaf through global counters took 222 us at 128^3; climbing on from
@@ -421,7 +423,7 @@ constexpr int kUpBlock = 512;
 
 template <bool COMP>
 constexpr int upward_smem() {
-    return (int)((COMP ? 14 : 10) * 2 * kUpBlock * sizeof(float) + 5 * kUpBlock * sizeof(int32_t));
+    return (int)((COMP ? 14 : 10) * 2 * kUpBlock * sizeof(float) + 6 * kUpBlock * sizeof(int32_t));
 }
 
 template <bool COMP>
@@ -438,7 +440,8 @@ __global__ void __launch_bounds__(kUpBlock) k_upward(const float *__restrict__ p
     int32_t *s_cnt = reinterpret_cast<int32_t *>(s_val + (COMP ? 14 : 10) * W);  // arrivals
     int32_t *s_who = s_cnt + kUpBlock;                                            // the first to arrive
     int32_t *s_l = s_who + kUpBlock, *s_r = s_l + kUpBlock, *s_p = s_r + kUpBlock;  // topology
-    __shared__ int s_left;                                                        // nodes left
+    int32_t *s_list = s_p + kUpBlock;  // nodes left, + 1: each thread climbs once, so at most one a leaf
+    __shared__ int s_left;
     const int64_t m_nodes = 2 * n - 1;
     const int t = threadIdx.x;
     const int64_t b0 = blockIdx.x * (int64_t)kUpBlock, i = b0 + t;
@@ -495,13 +498,13 @@ __global__ void __launch_bounds__(kUpBlock) k_upward(const float *__restrict__ p
         int32_t p = parents[curr];
         for (;;) {
             if (p == -1) break;  // the whole tree lies in the block
-            if (p < 0 || p >= m_nodes) {
+            if (p < n || p >= m_nodes) {  // a parent is an internal node
                 set_flag(status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
-            const int ps = p < n ? -1 : slot_of(p);
+            const int ps = slot_of(p);
             if (ps < 0) {
-                counts[b0 + atomicAdd(&s_left, 1)] = (int32_t)curr + 1;
+                s_list[atomicAdd(&s_left, 1)] = (int32_t)curr + 1;
                 break;
             }
             const int pk = ps - kUpBlock;
@@ -530,6 +533,7 @@ __global__ void __launch_bounds__(kUpBlock) k_upward(const float *__restrict__ p
         }
     }
     __syncthreads();
+    if (node < m_nodes && s_cnt[t] == 1) s_list[atomicAdd(&s_left, 1)] = s_who[t] + 1;
     // one array after the other, its floats on consecutive threads
     const auto write = [&](int base, int64_t first, int64_t end, bool leaf) {
         const int k = (int)min((int64_t)kUpBlock, end - first);  // nodes first .. first + k
@@ -549,7 +553,8 @@ __global__ void __launch_bounds__(kUpBlock) k_upward(const float *__restrict__ p
     write(0, b0, n, true);
     write(kUpBlock, n + b0, m_nodes, false);
     if (node < m_nodes && s_cnt[t] >= 2) counts[node] = 2;
-    if (node < m_nodes && s_cnt[t] == 1) counts[b0 + atomicAdd(&s_left, 1)] = s_who[t] + 1;
+    __syncthreads();
+    if (i < n) counts[i] = t < s_left ? s_list[t] : 0;
 }
 
 template <bool COMP>
@@ -562,8 +567,8 @@ __global__ void __launch_bounds__(256) k_upward_rest(const int32_t *__restrict__
     const int64_t curr = (int64_t)counts[i] - 1;
     if (curr < 0) return;
     counts[i] = 0;
-    climb_global<COMP>(A, curr, parents[curr], load_node_acc<COMP>(A, curr), children, parents, counts,
-                       2 * n - 1, status);
+    climb_global<COMP>(A, curr, parents[curr], load_node_acc<COMP>(A, curr), children, parents, counts, n,
+                       status);
 }
 
 // tree_kernels.py:193-214 normalize_com: inv = 1.0 / m in float64, com * inv

@@ -175,7 +175,9 @@ int cnb_validate_tree(const int32_t *children, const int32_t *parents, int64_t n
                       int32_t *scratch, int32_t *status, void *stream);
 
 /* src/kernels/tree_kernels.py:131-191 compute_multipoles(pos_x, pos_y, pos_z, mass,
- * children, parents, n_mass, n_com, n_min, n_max, counts).  n = bodies. */
+ * children, parents, n_mass, n_com, n_min, n_max, counts).  n = bodies.
+ * counts int32 [2N-1]: the internal nodes' counters must be zero on entry; the
+ * leaves' are scratch (any values on entry, zero afterwards). */
 int cnb_compute_multipoles(const float *px, const float *py, const float *pz,
                            const float *mass, const int32_t *children, const int32_t *parents,
                            float *n_mass, float *n_com, float *n_min, float *n_max,
@@ -189,7 +191,7 @@ int cnb_compute_multipoles(const float *px, const float *py, const float *pz,
  * the compensation terms (compensated mode only, else may be NULL).
  * root_f64 (device, 4 doubles: mass, CoM x, y, z; required in compensated
  * mode, optional in plain mode, where the float32 tree is left untouched)
- * receives the float64 root values.  counts must be zero on entry. */
+ * receives the float64 root values.  counts as for cnb_compute_multipoles. */
 int cnb_upward(const float *px, const float *py, const float *pz, const float *mass,
                const int32_t *children, const int32_t *parents, float *n_mass, float *n_com,
                float *n_min, float *n_max, float *n_err, int32_t *counts, int64_t n, int mode,
