@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
             soft2 = bp.y * bp.y;
             th2d = (double)th * (double)th;
         }
-        soft2 = fmaxf(soft2, kMinSoft2);
+        soft2 = normal_soft2(soft2);
         if (P.theta_per_bucket) {
             th = P.theta_per_bucket[g];
             th2d = (double)th * (double)th;

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(WARPS * 32, law_warps<LAW>() / WARPS) k_forces
             soft2 = bp.y * bp.y;
             slab_mass = bp.z;
         }
-        soft2 = fmaxf(soft2, kMinSoft2);
+        soft2 = normal_soft2(soft2);
         if (P.theta_per_bucket) th = P.theta_per_bucket[g];
         const float th2 = th * th;
 

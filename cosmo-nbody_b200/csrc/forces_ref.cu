@@ -11,12 +11,9 @@
 // reference (float32 node data, `round()` promoting the displacement);
 // T = float is the float32 form.  The reference's shared-memory copy of the
 // top 256 nodes only mirrors node data and is not needed for the result.
-#include <math.h>
-
 #include <type_traits>
 
 #include "grouped.cuh"
-
 
 namespace cnb {
 
@@ -412,7 +409,7 @@ int launch_exact_walk(const GroupedParams &P, cudaStream_t st) {
     R.rec = P.rec;
     R.theta_sq = P.theta * P.theta;
     R.G = P.G;
-    R.soft2 = fmaxf(P.soft2, kMinSoft2);
+    R.soft2 = normal_soft2(P.soft2);
     R.box = P.box;
     R.m_nodes = P.m_nodes;
     return forces_walk<float, true, true>(P.px, P.py, P.pz, R, P.theta_sq, P.force, nullptr, P.root, 0,
@@ -426,7 +423,7 @@ static int forces_ref(const float *px, const float *py, const float *pz, RefTree
     R.theta_sq = (T)(theta * theta);
     R.G = (T)G;
     R.soft2 = (T)(soft * soft);
-    if (sizeof(T) == 4) R.soft2 = R.soft2 > (T)kMinSoft2 ? R.soft2 : (T)kMinSoft2;
+    if (sizeof(T) == 4) R.soft2 = normal_soft2((float)R.soft2);
     R.box = (T)box;
     R.m_nodes = 2 * n - 1;
     if (count > n - off) count = n - off;

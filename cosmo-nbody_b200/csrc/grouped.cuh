@@ -85,6 +85,10 @@ constexpr float kRelMargin = 4e-6f;
 // for every pair.  Against rsqrtf: bucket test 128^3 2.30 -> 2.01 ms, exact test
 // 4.74 -> 4.48, periodic law 4.75 -> 4.46, float32 per-body walk 6.78 -> 6.22 ms.
 constexpr float kMinSoft2 = 1.17549435e-38f;
+// eps^2 raised to kMinSoft2; a NaN stays one, and reaches the forces and the status word
+__host__ __device__ __forceinline__ float normal_soft2(float soft2) {
+    return soft2 < kMinSoft2 ? kMinSoft2 : soft2;
+}
 __device__ __forceinline__ float rsqrt_normal(float q) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
