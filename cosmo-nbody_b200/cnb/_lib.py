@@ -35,6 +35,7 @@ MAC_REF_X_BUCKET = 3
 SORT_FULL = 0
 SORT_ADAPTIVE = 1
 SORT_NEAR_CAP = 2048
+EXACT_WALK_BODIES = 98304   # CNB_EXACT_WALK_BODIES
 PREC_F32 = 0
 PREC_F64 = 1
 UPWARD_PLAIN = 0

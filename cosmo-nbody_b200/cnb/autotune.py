@@ -44,6 +44,9 @@ def tune(engine, shapes=SHAPES, supers=SUPERS, reps=3, use_cache=True, save=True
     """Pick the fastest (bodies_per_lane, block_warps, super-bucket size) for
     `engine` (grouped mode, tree already built by forces_only/step).  Returns
     a report dict."""
+    if engine.walks_by_groups():   # one kernel, whatever the shape: nothing to choose or to remember
+        return {"shape": [engine.bodies_per_lane, engine.block_warps, engine.super_bodies], "ms": {},
+                "cached": False}
     key = _key(engine)
     if engine.mac not in (0, 3):   # the two-level walk exists for the reference test only
         supers = (0,)

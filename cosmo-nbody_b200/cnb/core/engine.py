@@ -121,6 +121,14 @@ class SimulationEngine:
         # the tree build makes the super-bucket table too
         self.tree_manager.set_super_table(self.super_ws, super_bodies)
 
+    def walks_by_groups(self):
+        """True when the force stage walks by groups of bodies, whatever the
+        launch shape and the super-bucket size (small systems, the reference's
+        test)."""
+        return (self.force_mode == "grouped" and self.mac == _lib.MAC_REF_X and
+                self.state.n <= _lib.EXACT_WALK_BODIES and self.controller is None and
+                self.theta_per_group is None)
+
     def _stream(self):
         return int(torch.cuda.current_stream(self.state.device).cuda_stream)
 
@@ -165,7 +173,7 @@ class SimulationEngine:
                           self.bucket_inter.data_ptr() if self.bucket_inter is not None else None,
                           self.stats.data_ptr(), status, st)
                 return
-            if self.super_ws is not None and tpg is None:
+            if self.super_ws is not None and tpg is None and not self.walks_by_groups():
                 # NULL ranges and parents: the super-bucket table was built with the tree
                 # (otherwise, e.g. after a change of super_bodies, the call builds it)
                 built = tm.super_table_current

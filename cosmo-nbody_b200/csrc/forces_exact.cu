@@ -790,16 +790,18 @@ static int launch_exact_shape(GroupedParams &P, cudaStream_t st) {
 
 static int g_test_spill_every = 0;  // cnb_exact_test_spill
 
-// Systems of at most this many bodies take the walk by groups (forces_ref.cu):
-// their few hundred buckets leave most warps of the chip idle while each is a
-// serial walk of some 80 000 instructions.  Measured, theta 0.5, an even and a
-// clustered state (us, the faster bucket form against groups): 20 000 bodies
-// 160 and 208 / 87 and 95, 65 536 247 and 322 / 253 and 263, 98 000 312 and 396 /
-// 333 and 396, 131 072 364 and 510 / 470 and 533.
-constexpr int64_t kWalkBodies = 98304;
-
+// Systems of at most CNB_EXACT_WALK_BODIES bodies take the walk by groups
+// (forces_ref.cu), super-buckets or not: their few hundred buckets leave most
+// warps of the chip idle while each is a serial walk of some 80 000 instructions.  Measured on even and clustered states at theta 0.4, 0.5,
+// 0.7 and 0.9 (us at 0.5, the fastest of six bucket shapes, one and two levels /
+// groups; in brackets the geometric mean over all states and angles of groups
+// against buckets): 20 000 bodies 162 and 184 / 80 and 90 (0.50), 50 000 226 and
+// 258 / 184 and 207 (0.79), 65 536 229 and 285 / 238 and 262 (0.96), 80 000 264 and
+// 365 / 283 and 315 (0.94), 98 304 342 and 401 / 365 and 391 (1.00), 131 072 377 and
+// 478 / 487 and 526 (1.15).  Even states at small angles cross earlier (0.4: between
+// 50 000 and 65 536), clustered ones and large angles later.
 int launch_exact(GroupedParams &P, int bodies_per_lane, int block_warps, cudaStream_t st) {
-    if (P.n <= kWalkBodies && !P.box_roots && !P.theta_per_bucket) return launch_exact_walk(P, st);
+    if (P.n <= CNB_EXACT_WALK_BODIES && !P.box_roots && !P.theta_per_bucket) return launch_exact_walk(P, st);
     P.test_spill_every = g_test_spill_every;
     switch (bodies_per_lane * 16 + block_warps) {
         case 16 + 2: return launch_exact_shape<1, 2>(P, st);

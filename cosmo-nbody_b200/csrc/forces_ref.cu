@@ -138,7 +138,7 @@ __device__ __noinline__ void walk_one(const RefTree<T> &R, int32_t root, float x
 // EXACT (T = float): the reference's float64 decisions on float32 forces, as
 // forces_exact.cu makes them (the test in float64 inside the band [lo, hi]
 // around s^2 / theta^2), without the reference's stack limit: the form the
-// grouped traversal takes on small systems (see kWalkBodies).
+// grouped traversal takes on small systems (CNB_EXACT_WALK_BODIES).
 //
 // Bound by the instructions of a step (about 40 for 32 pairs in float32); small
 // counts by the latency of the fetches, one round of 32 after the other.  One

@@ -347,6 +347,12 @@ int cnb_forces_grouped(const float *px, const float *py, const float *pz,
  * slot after its first round (0 = off; process-wide, not thread-safe). */
 int cnb_exact_test_spill(int every);
 
+/* With CNB_MAC_REF_X and one theta for all buckets systems of at most this many
+ * bodies are walked by groups of consecutive bodies instead of buckets: the
+ * same nodes, and faster there than either bucket form.  cnb_forces_two_level
+ * makes its lists there too, but walks without them: call cnb_forces_grouped. */
+#define CNB_EXACT_WALK_BODIES 98304
+
 /* Two-level form of cnb_forces_grouped (no reference counterpart; same
  * results as the one-level walk with the same mac, CNB_MAC_REF_X or
  * CNB_MAC_REF_X_BUCKET, up to float32 summation order).  The tree is cut
