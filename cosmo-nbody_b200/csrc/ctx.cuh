@@ -24,6 +24,9 @@ struct cnb_ctx {
     int32_t wait_limit = 0;          // look-back polls before a wait gives up (0: 2^22)
     int64_t withheld_tile = -1;      // one-sweep tile that never publishes its counts
     int64_t near_dest_bias = 0;      // added to the near-sorted path's R destinations
+    // cnb_ctx_inject_barrier_fault, the same for the persistent sort
+    int32_t barrier_wait_limit = 0;  // polls of a grid barrier before it gives up (0: 2^22)
+    int32_t withheld_block = -1;     // block that never arrives
     int persistent_blocks = 0;       // resident blocks of the persistent sort (0: not available)
     // grouped traversal scratch (grown on demand by cnb_forces_grouped)
     void *group_scratch = nullptr;

@@ -724,6 +724,13 @@ extern "C" int cnb_ctx_inject_sort_faults(cnb_ctx *ctx, int32_t wait_limit,
     return CNB_OK;
 }
 
+extern "C" int cnb_ctx_inject_barrier_fault(cnb_ctx *ctx, int32_t wait_limit, int32_t withheld_block) {
+    if (!ctx || wait_limit < 0 || withheld_block < -1) return CNB_E_INVALID_ARG;
+    ctx->barrier_wait_limit = wait_limit;
+    ctx->withheld_block = withheld_block;
+    return CNB_OK;
+}
+
 extern "C" int cnb_ctx_sort_stats(cnb_ctx *ctx, int64_t *out) {
     if (!ctx || !out) return CNB_E_INVALID_ARG;
     unsigned long long v[2];

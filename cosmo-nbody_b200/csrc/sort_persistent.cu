@@ -52,6 +52,7 @@ struct PersistentSort {
     const int32_t *skip;
     unsigned long long *stat;
     int wait_limit;
+    int withheld;  // tests: the block that never arrives (-1: none)
 };
 
 // Waits until every block has arrived `target` / gridDim.x times; false when
@@ -60,11 +61,11 @@ struct PersistentSort {
 __device__ __forceinline__ bool grid_wait(const PersistentSort &P, uint32_t target, int *s_ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ok = 1;
+        int ok = (int)blockIdx.x != P.withheld;
         __threadfence();
-        atomicAdd(P.bar, 1u);
+        if (ok) atomicAdd(P.bar, 1u);
         int spins = 0;
-        while (*(volatile uint32_t *)P.bar < target) {
+        while (ok && *(volatile uint32_t *)P.bar < target) {
             if (++spins > P.wait_limit) {
                 set_flag(P.flags, CNB_FLAG_WAIT_LIMIT);
                 ok = 0;
@@ -305,7 +306,8 @@ int sort_pairs_persistent(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_
     P.flags = ctx->flags;
     P.skip = skip;
     P.stat = ctx->sort_stats ? ctx->sort_stats + 1 : nullptr;
-    P.wait_limit = 1 << 22;
+    P.wait_limit = ctx->barrier_wait_limit > 0 ? ctx->barrier_wait_limit : 1 << 22;
+    P.withheld = ctx->withheld_block;
     if (!arrivals && blocks > 1) CNB_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(uint32_t), st));
     void *args[] = {&P};
     const bool few = P.chunk <= kPThreads * kPItems;

@@ -108,6 +108,14 @@ int cnb_sort_pairs(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
 int cnb_ctx_inject_sort_faults(cnb_ctx *ctx, int32_t wait_limit, int64_t withheld_tile,
                                int64_t near_dest_bias);
 
+/* The same hook for the full sort's one-launch form (cnb_sort_pairs outside
+ * stream capture, up to 14 336 keys a multiprocessor, while the hook above is
+ * off): wait_limit > 0 bounds every wait at its grid barriers at that many
+ * polls (0: the default 2^22); withheld_block >= 0 makes that block return at
+ * its first barrier without arriving, so the others wait until their limit,
+ * give up and raise CNB_FLAG_WAIT_LIMIT (-1: off).  Reset with (0, -1). */
+int cnb_ctx_inject_barrier_fault(cnb_ctx *ctx, int32_t wait_limit, int32_t withheld_block);
+
 /* No counterpart in the reference.  Sort mode of a context (default
  * CNB_SORT_FULL).  CNB_SORT_ADAPTIVE: cnb_sort_pairs with idx_in == NULL and
  * keys_in != keys_out first tries the near-sorted path -- keys that break
