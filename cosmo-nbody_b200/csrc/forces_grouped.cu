@@ -236,6 +236,8 @@ struct EwaldSums {
 // Warps per SM the registers are bounded for, by measurement: law 0 24 (77 registers: 128^3 bucket
 // test 2.00 ms; 28 and 20: 2.02, 2.06); law 1 28 (72 registers: 128^3 4.31 ms; left alone the
 // compiler takes 64 and 4.48 ms), law 2 20 (95 registers: 300k bodies 1.155 ms; 24: 1.23).
+// These are for one warp a bucket; the teams have the same bounds, under which law 1's of two and
+// four warps spill 64 and 40 bytes with 64-body buckets (other bounds not measured).
 template <int LAW> __host__ __device__ constexpr int law_warps() {
     return LAW == 1 ? 28 : LAW == 2 ? 20 : 24;
 }
@@ -1041,25 +1043,37 @@ static int launch_team_size(GroupedParams &P, int warps, cudaStream_t st) {
 // barriers a round, lanes without a node and its lists' remainders, so it is
 // wanted while its blocks (444, 1036 or 2072 resident for the periodic law, less
 // with quadrupoles) take about all buckets at once.  The minimum-image test's
-// chains are so long, and its stack so large, that two warps are never worse.
-// Measured (us, 1 / 2 / 4 / 8 warps, 64-body buckets; the lines of 32-body ones
-// lie at about half the bodies): periodic law 4 096 bodies 104 / 93 / 68 / 47,
-// 24 576 176 / 146 / 97 / 87, 65 536 217 / 167 / 162 / 179, 131 072 292 / 307 / 310 / 371;
-// quadrupoles 12 288 161 / 112 / 82 / 56, 16 384 175 / 128 / 92 / 93, 65 536 172 / 140 /
-// 146 / 216, 100 003 225 / 226 / 248 / 364; bucket test 24 576 142 / 110 / 72 / 71, 50 000 184 /
-// 136 / 121 / 135, 114 688 224 / 220 / 235 / 288; minimum image 12 288 687 / 722 / 444 /
-// 270, 50 000 2170 / 2159 / 1601 / 1591, 200 003 14.4 / 11.0 / 11.3 / 12.3 ms.
+// chains are so long that a team is never far behind.
+// Measured (us, 1 / 2 / 4 / 8 warps; the geometric mean of even and clustered states at
+// theta 0.5 and 0.8), 64-body buckets: bucket test 16 384 bodies 85 / 76 / 58 / 47, 24 576
+// 94 / 84 / 61 / 74, 49 152 124 / 94 / 92 / 114, 65 536 130 / 99 / 110 / 146, 98 304 144 / 138 /
+// 149 / 211, 114 688 144 / 147 / 164 / 232; periodic law 16 384 115 / 111 / 76 / 55, 24 576
+// 118 / 115 / 80 / 86, 49 152 168 / 130 / 120 / 136, 65 536 174 / 134 / 140 / 173, 81 920 174 /
+// 142 / 157 / 207, 98 304 185 / 194 / 191 / 249; quadrupoles 12 288 101 / 90 / 70 / 60, 16 384
+// 126 / 97 / 73 / 83, 32 768 117 / 100 / 86 / 123, 49 152 141 / 108 / 120 / 173, 81 920 154 / 153 /
+// 174 / 273, 98 304 167 / 177 / 207 / 336; minimum image 24 576 1563 / 1193 / 751 / 614, 49 152
+// 3171 / 2094 / 1543 / 1536, 65 536 3897 / 2539 / 2369 / 2442, 100 000 5602 / 4407 / 4236 / 4515
+// (clustered 200 003 14.4 / 11.0 / 11.3 / 12.3 ms).
+// 32-body buckets: bucket test 8 192 55 / 47 / 39 / 36, 12 288 57 / 51 / 43 / 56, 16 384 61 /
+// 53 / 45 / 62, 24 576 66 / 60 / 66 / 87, 32 768 72 / 64 / 74 / 106, 40 960 77 / 82 / 90 / 128,
+// 57 344 93 / 102 / 121 / 186; periodic law 8 192 70 / 63 / 49 / 42, 16 384 80 / 69 / 58 / 74,
+// 24 576 88 / 76 / 86 / 105, 40 960 98 / 85 / 103 / 156, 50 000 105 / 117 / 128 / 187; quadrupoles
+// 6 144 71 / 61 / 49 / 47, 16 384 81 / 70 / 66 / 97, 20 480 83 / 71 / 81 / 118, 32 768 87 / 86 / 101 /
+// 166; minimum image 16 384 853 / 688 / 452 / 419, 24 576 1195 / 975 / 717 / 722, 65 536 3434 /
+// 2958 / 2908 / 3086, 100 000 5343 / 5451 / 5499 / 5952.
+// The last limits lie up to a tenth past the crossing: a team's stack never drops
+// a node, one warp's 512 entries may.
 static int team_warps(const GroupedParams &P, int bodies_per_lane) {
     const bool wide = bodies_per_lane == 2;
     struct { int64_t eight, four, two; } most;  // bodies
     if (P.mac == CNB_MAC_PERIODIC)
-        most = wide ? decltype(most){49152, 65536, INT64_MAX} : decltype(most){12288, 49152, INT64_MAX};
+        most = wide ? decltype(most){49152, 131072, INT64_MAX} : decltype(most){24576, 65536, INT64_MAX};
     else if (P.mac != CNB_MAC_EWALD)
-        most = wide ? decltype(most){24576, 49152, 114688} : decltype(most){8192, 24576, 57344};
+        most = wide ? decltype(most){20480, 57344, 114688} : decltype(most){10240, 20480, 57344};
     else if (P.quad)
-        most = wide ? decltype(most){12288, 49152, 98304} : decltype(most){6144, 20480, 32768};
+        most = wide ? decltype(most){14336, 40960, 98304} : decltype(most){7168, 18432, 32768};
     else
-        most = wide ? decltype(most){24576, 65536, 98304} : decltype(most){8192, 32768, 40960};
+        most = wide ? decltype(most){20480, 57344, 98304} : decltype(most){10240, 20480, 45056};
     return P.n <= most.eight ? 8 : P.n <= most.four ? 4 : P.n <= most.two ? 2 : 1;
 }
 

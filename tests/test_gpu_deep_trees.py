@@ -63,9 +63,9 @@ def test_exact_decisions_by_groups(n, theta):
 
 # per law and bucket width a size for teams of eight, four and two warps
 TEAMS = {("bucket", 2): (20000, 40000, 70000), ("bucket", 1): (8000, 20000, 40000),
-         ("periodic", 2): (20000, 59145, 70000), ("periodic", 1): (12000, 40000, 59145),
-         ("ewald", 2): (20000, 59145, 70000), ("ewald", 1): (8000, 30000, 40000),
-         ("quad", 2): (12000, 40000, 70000), ("quad", 1): (6000, 20000, 30000)}
+         ("periodic", 2): (20000, 70000, 140000), ("periodic", 1): (12000, 40000, 70000),
+         ("ewald", 2): (20000, 50000, 70000), ("ewald", 1): (8000, 20000, 40000),
+         ("quad", 2): (12000, 40000, 70000), ("quad", 1): (6000, 18000, 30000)}
 
 
 @pytest.mark.parametrize("theta", [0.0, 0.1, 0.2])
