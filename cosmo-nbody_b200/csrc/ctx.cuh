@@ -51,6 +51,7 @@ int sort_pairs_onesweep(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_ou
 // zeroed word for its barriers, or null (it zeroes one itself).
 int persistent_blocks();
 int64_t persistent_max(const cnb_ctx *ctx);
+constexpr int kNotResident = 1;  // nothing was launched: the stream's part of the GPU holds too few blocks
 int sort_pairs_persistent(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_out,
                           const uint32_t *idx_in, uint32_t *perm_out, int64_t n, int key_bits,
                           cudaStream_t st, const int32_t *skip, uint32_t *arrivals);

@@ -657,14 +657,16 @@ extern "C" int cnb_sort_pairs(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *k
     CNB_CUDA(cudaStreamIsCapturing(st, &cs));
     const bool capturing = cs == cudaStreamCaptureStatusActive;
     // the full sort: one cooperative launch, or the one-sweep launches when the stream is being
-    // captured or a fault of theirs is injected
+    // captured, a fault of theirs is injected, or the stream's part of the GPU does not hold all
+    // blocks of the one launch
     const bool persistent = !capturing && n > 0 && n <= cnb::persistent_max(ctx) && ctx->wait_limit == 0 &&
                             ctx->withheld_tile < 0;
     const auto full_sort = [&](const uint32_t *idx) {
-        return persistent ? cnb::sort_pairs_persistent(ctx, keys_in, keys_out, idx, perm_out, n, key_bits,
-                                                       st, skip, arrivals)
-                          : cnb::sort_pairs_onesweep(ctx, keys_in, keys_out, idx, perm_out, n, key_bits, st,
-                                                     skip);
+        const int rc = persistent ? cnb::sort_pairs_persistent(ctx, keys_in, keys_out, idx, perm_out, n,
+                                                               key_bits, st, skip, arrivals)
+                                  : cnb::kNotResident;
+        return rc != cnb::kNotResident
+                   ? rc : cnb::sort_pairs_onesweep(ctx, keys_in, keys_out, idx, perm_out, n, key_bits, st, skip);
     };
     if (!(ctx->sort_mode == CNB_SORT_ADAPTIVE && n > 0 && idx_in == nullptr && keys_in != keys_out))
         return full_sort(idx_in);

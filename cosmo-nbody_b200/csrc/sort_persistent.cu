@@ -311,9 +311,14 @@ int sort_pairs_persistent(cnb_ctx *ctx, const uint64_t *keys_in, uint64_t *keys_
     if (!arrivals && blocks > 1) CNB_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(uint32_t), st));
     void *args[] = {&P};
     const bool few = P.chunk <= kPThreads * kPItems;
-    CNB_CUDA(cudaLaunchCooperativeKernel(
+    const cudaError_t e = cudaLaunchCooperativeKernel(
         few ? (const void *)k_sort_persistent<kPItems> : (const void *)k_sort_persistent<kPItemsMost>,
-        dim3((unsigned)blocks), dim3(kPThreads), args, persistent_smem(few ? kPItems : kPItemsMost), st));
+        dim3((unsigned)blocks), dim3(kPThreads), args, persistent_smem(few ? kPItems : kPItemsMost), st);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kNotResident;
+    }
+    CNB_CUDA(e);
     return launch_status();
 }
 

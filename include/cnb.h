@@ -110,7 +110,7 @@ int cnb_ctx_inject_sort_faults(cnb_ctx *ctx, int32_t wait_limit, int64_t withhel
 
 /* The same hook for the full sort's one-launch form (cnb_sort_pairs outside
  * stream capture, up to 14 336 keys a multiprocessor, while the hook above is
- * off): wait_limit > 0 bounds every wait at its grid barriers at that many
+ * off and the stream has the whole GPU): wait_limit > 0 bounds every wait at its grid barriers at that many
  * polls (0: the default 2^22); withheld_block >= 0 makes that block return at
  * its first barrier without arriving, so the others wait until their limit,
  * give up and raise CNB_FLAG_WAIT_LIMIT (-1: off).  Reset with (0, -1). */

@@ -70,6 +70,57 @@ def test_a_short_limit_alone_sorts_or_reports():
         _lib.load().cnb_ctx_destroy(ctx)
 
 
+PART = r"""
+import ctypes as C, sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+from cnb import _lib
+n = 300007
+keys = np.random.default_rng(2).integers(0, 1 << 63, n, dtype=np.uint64)
+K = torch.from_numpy(keys).cuda()
+ko, po = torch.zeros_like(K), torch.zeros(n, dtype=torch.int32, device="cuda")
+status = torch.zeros(1, dtype=torch.int32, device="cuda")
+want = np.argsort(keys, kind="stable")
+torch.cuda.synchronize()
+try:
+    part = torch.cuda.GreenContext.create(16, 0)
+except RuntimeError as e:
+    print("no green contexts:", e)
+    sys.exit(0)
+for mode in (_lib.SORT_FULL, _lib.SORT_ADAPTIVE):
+    ctx = C.c_void_p()
+    _lib.call("cnb_ctx_create", n, C.byref(ctx))
+    _lib.call("cnb_ctx_set_sort_mode", ctx, mode)
+    torch.cuda.synchronize()
+    part.set_context()
+    s = torch.cuda.Stream()
+    _lib.call("cnb_sort_pairs", ctx, K.data_ptr(), ko.data_ptr(), None, po.data_ptr(), n, 63, int(s.cuda_stream))
+    _lib.call("cnb_ctx_take_flags", ctx, status.data_ptr(), int(s.cuda_stream))
+    s.synchronize()
+    part.pop_context()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert (po.cpu().numpy() == want).all() and (ko.cpu().numpy() == keys[want]).all()
+    _lib.load().cnb_ctx_destroy(ctx)
+print("sorted")
+"""
+
+
+def test_a_stream_with_part_of_the_gpu():
+    """A stream of a green context of 16 multiprocessors does not hold the
+    persistent sort's blocks: the one-sweep launches sort there.  (In a process
+    of its own: torch keeps a pool of streams that would belong to the part.)"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", PART, os.path.join(root, "cosmo-nbody_b200")],
+                       capture_output=True, text=True, timeout=300)
+    if "no green contexts" in r.stdout:
+        pytest.skip(r.stdout.strip())
+    assert r.returncode == 0 and "sorted" in r.stdout, r.stderr[-2000:]
+
+
 def test_arguments():
     from cnb import _lib
     lib = _lib.load()
