@@ -60,18 +60,36 @@ namespace cnb {
 // reached by the whole bucket (one word, the node) grow up from word 0,
 // entries reached by part of it (three words: node, mask low, mask high)
 // grow down from the end.  A round pops no more entries than the free words
-// can take back, so a walk that fills the region narrows to a depth-first one
-// and only a path some thirty levels deeper still is given up by the main pass
-// (it marks the bucket's record and writes no force for it); a second pass
-// walks those buckets again with a region of kXWordsRedo words, and drops what
-// does not fit there (CNB_FLAG_LIST_OVERFLOW).  Rounds are full until 480 of
-// the 640 words are used; the deepest use at theta = 0.5 on 128^3 and 256^3
-// Zel'dovich and evolved states (two-level walk included) is 607 words.
-// 640 against 864 words (and 2048 at small angles or with several boxes, as
-// one size used to need): theta 0.3 500k bodies 4.72 -> 4.35 ms, 16 boxes
-// 1.48 -> 1.37; 512 and 496 are no faster.
-constexpr int kXWords = 640;       // main pass
-constexpr int kXWordsRedo = 4096;  // the buckets a main pass gave up on
+// can take back, so it is full until 160 words are left and narrows from there.
+// A walk that goes on in rounds of fewer than kXLeast entries would crawl, so
+// after kXNarrow of them (or without room for one) the main pass gives the
+// bucket up: it marks the bucket's record and writes no force for it.  A second
+// pass walks those buckets again with a region of kXWordsRedo words, by the main
+// pass's rule up to where that gave up and in full rounds from there.  Its last
+// kXDeep words are left to rounds of one entry, a depth-first walk: it takes at
+// most five words where part of the bucket first opens a node and three a level
+// from there, and a radix tree over 64-bit keys has at most 64 + 32 levels, so
+// only a caller's own, deeper tree can overflow the region
+// (CNB_FLAG_LIST_OVERFLOW).
+//
+// The main pass's region, by what a walk needs and what its words cost in warps
+// and cache: at theta = 0.5 on 128^3 and 256^3 Zel'dovich and evolved states (two
+// levels included) the deepest use is 607 words; cusps of 64 levels use 400 to
+// 800 at theta 0.5 and above, 1200 to 1500 at 0.3, 2000 at 0.1.  Measured (us,
+// regions of 640 / 864 / 1280 / 1536 / 2048 words): 500k Zel'dovich bodies theta
+// 0.3 3960 / - / 4000 / 4140 / 4300, 120k bodies in a cusp, 64-body buckets, theta
+// 0.5 880 / 555, theta 0.3 2370 / - / 1270 / 1340 / 1350, theta 0.25 - / - / 3010 / 1690,
+// theta 0.1 9290 / - / 9720 / - / 5360; 16 boxes 1405 / 1450; 2M bodies theta 0.5 the same
+// within 0.5 %.  Without the second pass's share (32 neighbouring records a warp,
+// so that a cusp's buckets fell to a few warps) and the limit on narrow rounds
+// 640 words for every angle took 14.5 ms at theta 0.3 and 82 ms at 0.1.
+constexpr int kXWords = 640;        // one body a lane; several boxes
+constexpr int kXWordsTwo = 864;     // two bodies a lane
+constexpr int kXWordsWide = 1280;   // theta below 0.4
+constexpr int kXWordsWidest = 2048; // theta below 0.25
+constexpr int kXWordsRedo = 4096;   // the buckets a main pass gave up on
+constexpr int kXLeast = 8, kXNarrow = 16, kXDeep = 320;
+static_assert(kXDeep >= 5 + 3 * (64 + 32), "three words a level for a depth-first walk");
 template <int XW> __device__ __forceinline__ int part_word(int k) { return XW - 3 * (k + 1); }
 
 // per-warp shared memory: the masked list (packed for two bodies per lane), the
@@ -374,14 +392,16 @@ __device__ __forceinline__ void flush32(float4 *lst, uint2 *msk, int &cnt, int l
 }
 
 // REDO false: the main pass over every bucket (work counter); true: the
-// buckets a main pass gave up on (bucket record's fourth word = 1), found by
-// a strided scan of the table and cleared when done.
+// buckets a main pass with MAIN words gave up on (bucket record's fourth word =
+// 1), found by a strided scan of the table and cleared when done.
 // Twenty warps per SM with two bodies per lane, 28 with one (24 in blocks of
 // eight).  Two bodies want their registers: bounded for 22 or 24 warps the
 // kernel is 2 % faster to 6 % slower at 2M bodies and 8 to 13 % slower at 300k.
-// One body leaves room: 128^3 one level 5.72 (16 warps) -> 4.88 ms (24).
-template <int BPL, int WARPS, int XW, bool REDO, bool TEST = false>
-__global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_forces_exact(GroupedParams P) {
+// One body leaves room: 128^3 one level 5.72 (16 warps) -> 4.88 ms (24).  The redo
+// pass's region leaves ten warps their shared memory.
+template <int BPL, int WARPS, int XW, bool REDO, bool TEST = false, int MAIN = XW>
+__global__ void __launch_bounds__(WARPS * 32, (REDO ? 10 : BPL == 2 ? 20 : 28) / WARPS)
+    k_forces_exact(GroupedParams P) {
     static_assert(BPL == 1 || BPL == 2, "one or two bodies per lane");
     extern __shared__ __align__(16) unsigned char x_smem[];
     constexpr int EW = entry_width<BPL>();
@@ -405,22 +425,24 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
     const float half_box = 0.5f * P.box;
 
     int4 *table = reinterpret_cast<int4 *>(P.ws + 4);  // the bucket records (P.buckets)
-    // redo: this warp's share of the table, 32 records at a time (lane l reads record
-    // chunk + l); marked holds the records of the chunk still to walk
-    int chunk = (blockIdx.x * WARPS + wib) * 32;
+    // redo: this warp's share of the table, every `warps`-th record, 32 of them at a time (lane l
+    // reads record chunk + l * warps: the records of a dense part of the system lie together);
+    // marked holds those still to walk
+    const int warps = gridDim.x * WARPS;
+    int chunk = blockIdx.x * WARPS + wib;
     uint32_t marked = 0u;
     for (;;) {
         int g = 0;
         if (REDO) {
             while (marked == 0u && chunk < n_buckets) {
-                const int r = chunk + lane;
+                const int r = chunk + lane * warps;
                 marked = __ballot_sync(0xffffffffu, r < n_buckets && table[r].w == 1);
-                if (marked == 0u) chunk += gridDim.x * WARPS * 32;
+                if (marked == 0u) chunk += 32 * warps;
             }
             if (marked == 0u) break;
-            g = chunk + __ffs(marked) - 1;
+            g = chunk + (__ffs(marked) - 1) * warps;
             marked &= marked - 1u;
-            if (marked == 0u) chunk += gridDim.x * WARPS * 32;
+            if (marked == 0u) chunk += 32 * warps;
         } else {
             if (lane == 0) g = atomicAdd(P.ws + 1, 1);
             g = __shfl_sync(0xffffffffu, g, 0);
@@ -525,25 +547,37 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
         }
         if (!seeded && lane == 0) stack[0] = root;
         __syncwarp();
-        int64_t rounds = 0;
+        uint32_t rounds = 0;
+        int narrow = 0;     // rounds of fewer than kXLeast entries
+        bool wide = false;  // redo: the main pass has given up here
         while ((top > 0 || ptop > 0) && !spill) {
             // a valid tree pushes every node at most once per bucket
-            if (++rounds > P.m_nodes) {
+            if (++rounds > (uint32_t)P.m_nodes) {
                 if (lane == 0) set_flag(P.status, CNB_FLAG_BAD_TOPOLOGY);
                 break;
             }
             // A popped entry leaves at most five words more than it took (a whole-bucket entry
             // opened by part of the bucket: one word becomes two (node, mask) entries), so
-            // popping a fifth of the free words never overflows the region; a full one is spilt.
-            // The redo pass goes by the main pass's region for as long as that lasts: the same
-            // order of nodes, so the same sums.
+            // popping a fifth of the free words never overflows the region.
+            // The redo pass goes by the main pass's region (MAIN) for as long as that lasts: the
+            // same order of nodes, so the same sums.
             const int used = top + 3 * ptop;
-            int room = ((kXWords - used) * 51) >> 8;
-            if (REDO && room <= 0) room = ((XW - used) * 51) >> 8;
-            if (room <= 0) {
-                if (REDO) overflow = true;
-                spill = true;
-                break;
+            int room = ((MAIN - used) * 51) >> 8;
+            if (room < kXLeast && !(REDO && wide)) {
+                if (room <= 0 || ++narrow > kXNarrow) {
+                    if (!REDO) {
+                        spill = true;
+                        break;
+                    }
+                    wide = true;
+                }
+            }
+            if (REDO && wide) {
+                if (used + 5 > XW) {
+                    overflow = spill = true;
+                    break;
+                }
+                room = max(((XW - kXDeep - used) * 51) >> 8, 1);
             }
             // part-bucket entries first (they keep the second stack short)
             const int k1 = min(ptop, min(32, room));
@@ -721,7 +755,7 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
             if (TEST && rounds == 1 && g % P.test_spill_every == 0) spill = true;
         }
         if (!REDO && spill) {
-            // the stacks would meet: no force and no counts from this pass; the redo
+            // given up: no force and no counts from this pass; the redo
             // pass walks it again
             if (lane == 0) table[g].w = 1;
             __syncwarp();
@@ -763,29 +797,35 @@ __global__ void __launch_bounds__(WARPS * 32, (BPL == 2 ? 20 : 28) / WARPS) k_fo
     if (lane == 0) atomicMax(P.ws + 2, max_top);
 }
 
-template <int BPL, int WARPS, int XW, bool REDO, bool TEST = false>
+template <int BPL, int WARPS, int XW, bool REDO, bool TEST = false, int MAIN = XW>
 static int launch_exact_pass(GroupedParams &P, cudaStream_t st) {
     const size_t smem = exact_smem<BPL>(WARPS, XW);
-    CNB_CUDA(cudaFuncSetAttribute(k_forces_exact<BPL, WARPS, XW, REDO, TEST>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const auto kernel = k_forces_exact<BPL, WARPS, XW, REDO, TEST, MAIN>;
+    CNB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_forces_exact<BPL, WARPS, XW, REDO, TEST>,
-                                                  WARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, WARPS * 32, smem);
     // persistent grid: the work counter (main pass) or the table scan (redo) hands out buckets
-    k_forces_exact<BPL, WARPS, XW, REDO, TEST>
-        <<<kSMs * (per_sm > 0 ? per_sm : 1), WARPS * 32, smem, st>>>(P);
+    kernel<<<kSMs * (per_sm > 0 ? per_sm : 1), WARPS * 32, smem, st>>>(P);
     return launch_status();
+}
+
+template <int BPL, int WARPS, int MAIN>
+static int launch_exact_region(GroupedParams &P, cudaStream_t st) {
+    if (P.test_spill_every > 0)  // tests: the main pass gives up on every n-th bucket
+        CNB_TRY((launch_exact_pass<BPL, WARPS, MAIN, false, true>(P, st)));
+    else
+        CNB_TRY((launch_exact_pass<BPL, WARPS, MAIN, false>(P, st)));
+    // the buckets it gave up on, if any (otherwise every warp scans its share of the
+    // bucket table and returns)
+    return launch_exact_pass<BPL, 2, kXWordsRedo, true, false, MAIN>(P, st);
 }
 
 template <int BPL, int WARPS>
 static int launch_exact_shape(GroupedParams &P, cudaStream_t st) {
-    if (P.test_spill_every > 0)  // tests: the main pass gives up on every n-th bucket
-        CNB_TRY((launch_exact_pass<BPL, WARPS, kXWords, false, true>(P, st)));
-    else
-        CNB_TRY((launch_exact_pass<BPL, WARPS, kXWords, false>(P, st)));
-    // the buckets it gave up on, if any (otherwise every warp scans its share of the
-    // bucket table and returns)
-    return launch_exact_pass<BPL, 2, kXWordsRedo, true>(P, st);
+    if (P.box_roots) return launch_exact_region<BPL, WARPS, kXWords>(P, st);
+    if (P.theta < 0.25f) return launch_exact_region<BPL, WARPS, kXWordsWidest>(P, st);
+    if (P.theta < 0.4f) return launch_exact_region<BPL, WARPS, kXWordsWide>(P, st);
+    return launch_exact_region<BPL, WARPS, BPL == 2 ? kXWordsTwo : kXWords>(P, st);
 }
 
 static int g_test_spill_every = 0;  // cnb_exact_test_spill

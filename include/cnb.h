@@ -280,8 +280,8 @@ int cnb_build_tree_ranges(const uint64_t *codes, int32_t *children, int32_t *par
  * 16-byte aligned) is int32 [4 + 4N]: [0] bucket count, [1] work counter,
  * [2] deepest node stack seen by the traversal (entries; for CNB_MAC_REF_X
  * words of its stack region, one per whole-bucket entry and three per
- * part-bucket entry: 640 words in the main pass, 4096 when a bucket is walked
- * again; small systems, walked by groups of bodies or by teams of warps whose
+ * part-bucket entry: 640 to 2048 words in the main pass, by theta and
+ * bodies_per_lane, 4096 when a bucket is walked again; small systems, walked by groups of bodies or by teams of warps whose
  * size does not follow block_warps: entries of a group or team), [3] the bodies' (index + 1)
  * summed over all buckets modulo 2^32 (N(N+1)/2 when the buckets tile the
  * bodies once; cnb_upward_table_buckets flags CNB_FLAG_BAD_TOPOLOGY
@@ -347,10 +347,10 @@ int cnb_forces_grouped(const float *px, const float *py, const float *pz,
                        unsigned long long *stats, int32_t *status, void *stream);
 
 /* With CNB_MAC_REF_X the traversal runs in two passes: the main pass gives up
- * on a bucket whose node stacks would outgrow its shared-memory region (it
- * marks the bucket record's fourth word and writes no force for it), and a
- * second pass walks only the marked buckets again with a region 6.4 times as
- * large (two passes with the same nodes: the same forces).  Tests only:
+ * on a bucket whose node stacks outgrow its shared-memory region (it marks the
+ * bucket record's fourth word and writes no force for it), and a second pass
+ * walks only the marked buckets again with a larger region (two passes with the
+ * same nodes: the same forces).  Tests only:
  * cnb_exact_test_spill(k) makes the main pass give up on every k-th bucket
  * slot after its first round (0 = off; process-wide, not thread-safe). */
 int cnb_exact_test_spill(int every);
