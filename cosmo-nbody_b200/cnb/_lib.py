@@ -36,6 +36,7 @@ SORT_FULL = 0
 SORT_ADAPTIVE = 1
 SORT_NEAR_CAP = 2048
 EXACT_WALK_BODIES = 98304   # CNB_EXACT_WALK_BODIES
+EXACT_WALK_BODIES_SMALL_ANGLE = 24576   # below theta 0.4
 PREC_F32 = 0
 PREC_F64 = 1
 UPWARD_PLAIN = 0

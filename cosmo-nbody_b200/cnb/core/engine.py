@@ -125,9 +125,10 @@ class SimulationEngine:
         """True when the force stage walks by groups of bodies, whatever the
         launch shape and the super-bucket size (small systems, the reference's
         test)."""
-        return (self.force_mode == "grouped" and self.mac == _lib.MAC_REF_X and
-                self.state.n <= _lib.EXACT_WALK_BODIES and self.controller is None and
-                self.theta_per_group is None)
+        most = (_lib.EXACT_WALK_BODIES_SMALL_ANGLE if float(self.config.THETA) < 0.4
+                else _lib.EXACT_WALK_BODIES)
+        return (self.force_mode == "grouped" and self.mac == _lib.MAC_REF_X and self.state.n <= most and
+                self.controller is None and self.theta_per_group is None)
 
     def _stream(self):
         return int(torch.cuda.current_stream(self.state.device).cuda_stream)

@@ -839,9 +839,12 @@ static int g_test_spill_every = 0;  // cnb_exact_test_spill
 // 258 / 184 and 207 (0.79), 65 536 229 and 285 / 238 and 262 (0.96), 80 000 264 and
 // 365 / 283 and 315 (0.94), 98 304 342 and 401 / 365 and 391 (1.00), 131 072 377 and
 // 478 / 487 and 526 (1.15).  Even states at small angles cross earlier (0.4: between
-// 50 000 and 65 536), clustered ones and large angles later.
+// 50 000 and 65 536), clustered ones and large angles later; below theta 0.4 the
+// groups need a larger stack and the line is CNB_EXACT_WALK_BODIES_SMALL_ANGLE (see
+// forces_ref.cu).
 int launch_exact(GroupedParams &P, int bodies_per_lane, int block_warps, cudaStream_t st) {
-    if (P.n <= CNB_EXACT_WALK_BODIES && !P.box_roots && !P.theta_per_bucket) return launch_exact_walk(P, st);
+    const int64_t groups = P.theta < 0.4f ? CNB_EXACT_WALK_BODIES_SMALL_ANGLE : CNB_EXACT_WALK_BODIES;
+    if (P.n <= groups && !P.box_roots && !P.theta_per_bucket) return launch_exact_walk(P, st);
     P.test_spill_every = g_test_spill_every;
     switch (bodies_per_lane * 16 + block_warps) {
         case 16 + 2: return launch_exact_shape<1, 2>(P, st);

@@ -147,28 +147,37 @@ __device__ __noinline__ void walk_one(const RefTree<T> &R, int32_t root, float x
 // float64 2 097 152 37.3 -> 11.4 ms, 5 000 of 64 000 840 -> 80 us.
 //
 // The stack never fills on a radix tree.  A popped entry leaves at most one more
-// than it took, so popping a quarter of what is free below kRefWide keeps rounds
-// of several entries within kRefWide; from there on a round pops one, and a
-// depth-first walk holds at most an entry a level more.  The levels of a tree
-// over 64-bit keys, runs of equal ones split by index, are at most 64 + 32: the
-// kRefStack - kRefWide entries kept for it are more.  Only a caller's own,
-// deeper tree can fill the stack.
+// than it took, so popping a part of what is free below kRefDeep keeps rounds of
+// several entries below it; from there on a round pops one, and a depth-first
+// walk holds at most an entry a level more.  The levels of a tree over 64-bit
+// keys, runs of equal ones split by index, are at most 64 + 32: the kRefDeep
+// entries kept for it are more.  Only a caller's own, deeper tree can fill the stack.
+//
+// A full stack is slow, though: rounds of one node.  Walks at small angles open
+// far more, and on deep trees fill 512 entries, so EXACT takes 848 below theta
+// 0.4 (seven blocks an SM; 1024 leave six), and a sixteenth of the free ones a
+// round instead of a quarter (us, 512 / 848 entries / the faster bucket shape; a
+// cusp of 64 levels, then an even state): 5 000 bodies theta 0.1 1313 / 262 / 279, 170 /
+// 168 / 451, theta 0.3 70 / 70 / 136, 63 / 64 / 229; 20 000 theta 0.1 5162 / 1292 / 868, 1012 /
+// 1120 / 1387, theta 0.2 2326 / 590 / 497, 485 / 547 / 750, theta 0.3 1048 / 229 / 313, 236 /
+// 260 / 393.  30 000 bodies with 1024 entries against buckets: theta 0.2 702 / 551, 907 / 870,
+// theta 0.3 334 / 315, 426 / 451: the line between lies at 24 576
+// (CNB_EXACT_WALK_BODIES_SMALL_ANGLE).
 constexpr int kRefWarps = 4;
-constexpr int kRefStack = 512;   // entries of a warp's shared stack
-constexpr int kRefWide = kRefStack - 128;
+constexpr int kRefDeep = 128;
 constexpr int kRefDepth = 63;
-static_assert(kRefStack - kRefWide > 64 + 32, "a level each for a depth-first walk");
+static_assert(kRefDeep > 64 + 32, "a level each for a depth-first walk");
 
 // What a step reads of an entry, two 128-bit words: (com, w) and
 //   float:  (G m, sx^2 or -1 for a leaf, targets, 0)
 //   EXACT:  (lo, hi, s, targets), w the mass
 //   double: (sx^2 or -1, G m), w the targets
-template <typename T>
+template <int STACK, bool DEPTH>
 struct WalkSmem {
-    int2 stack[kRefStack];      // (node, targets)
+    int2 stack[STACK];  // (node, targets)
     float4 node[32];
     float4 more[32];
-    uint8_t depth[kRefStack];
+    uint8_t depth[DEPTH ? STACK : 1];
 };
 
 // The rare part of an EXACT test: d^2 inside the band around s^2 / theta^2 or
@@ -178,7 +187,8 @@ static __device__ __noinline__ int decide_f64(float s, double theta_sq, float dx
     return ((double)s * (double)s < theta_sq * d2 ? 1 : 0) | (d2 > 1e-7 ? 2 : 0);
 }
 
-template <typename T, int GROUP, bool TABLE, bool EXACT>
+// STACK: entries of a warp's shared stack
+template <typename T, int GROUP, bool TABLE, bool EXACT, int STACK>
 __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     const float *__restrict__ px, const float *__restrict__ py, const float *__restrict__ pz,
     RefTree<T> R, double theta_sq, float *__restrict__ force, const int32_t *__restrict__ root_idx,
@@ -186,9 +196,9 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     int32_t *status) {
     constexpr int SLOTS = 32 / GROUP;
     constexpr uint32_t kGroupMask = GROUP == 32 ? 0xffffffffu : (1u << (GROUP % 32)) - 1u;
-    __shared__ WalkSmem<T> smem[kRefWarps];
+    __shared__ WalkSmem<STACK, !EXACT> smem[kRefWarps];
     const int lane = threadIdx.x & 31;
-    WalkSmem<T> &S = smem[threadIdx.x >> 5];
+    WalkSmem<STACK, !EXACT> &S = smem[threadIdx.x >> 5];
     const uint32_t lt = (1u << lane) - 1u;
     const int64_t first = (blockIdx.x * (int64_t)kRefWarps + (threadIdx.x >> 5)) * GROUP;
     if (first >= count) return;
@@ -208,12 +218,12 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     uint32_t n_acc = 0;
     if (lane == 0) {
         S.stack[0] = make_int2(root, (int)(members == 32 ? 0xffffffffu : (1u << members) - 1u));
-        S.depth[0] = 0;
+        if (!EXACT) S.depth[0] = 0;
     }
     __syncwarp();
     while (top > 0) {
         // fewer as the stack fills, down to a depth-first walk
-        const int room = (kRefWide - top) >> 2;
+        const int room = (STACK - kRefDeep - top) >> (STACK > 512 ? 4 : 2);
         const int k = min(top, min(32, room > 1 ? room : 1));
         top -= k;
         popped += k;
@@ -309,10 +319,10 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
         const bool p1 = opened && ch.x != -1, p2 = opened && ch.y != -1;
         const uint32_t m1 = __ballot_sync(0xffffffffu, p1), m2 = __ballot_sync(0xffffffffu, p2);
         const int pushed = __popc(m1) + __popc(m2);
-        if (top + pushed > kRefStack || popped > R.m_nodes ||
+        if (top + pushed > STACK || popped > R.m_nodes ||
             (!EXACT && __any_sync(0xffffffffu, opened && depth >= kRefDepth))) {
             alone = true;
-            full = top + pushed > kRefStack;
+            full = top + pushed > STACK;
             break;
         }
         int at = top + __popc(m1 & lt) + __popc(m2 & lt);
@@ -365,7 +375,7 @@ __global__ void __launch_bounds__(kRefWarps * 32) k_forces_walk(
     if (!isfinite(fx) || !isfinite(fy) || !isfinite(fz)) set_flag(status, CNB_FLAG_NONFINITE);
 }
 
-template <typename T, int GROUP, bool TABLE, bool EXACT>
+template <typename T, int GROUP, bool TABLE, bool EXACT, int STACK>
 static int launch_walk(const float *px, const float *py, const float *pz, const RefTree<T> &R,
                        double theta_sq, float *force, const int32_t *root_idx, int32_t root_node,
                        int64_t off, int64_t count, unsigned long long *stats, int32_t *max_stack,
@@ -373,18 +383,18 @@ static int launch_walk(const float *px, const float *py, const float *pz, const 
     const int64_t per_block = (int64_t)kRefWarps * GROUP;
     const int64_t grid = (count + per_block - 1) / per_block;
     if (grid > INT32_MAX) return CNB_E_TOO_LARGE;
-    k_forces_walk<T, GROUP, TABLE, EXACT><<<(unsigned)grid, kRefWarps * 32, 0, st>>>(
+    k_forces_walk<T, GROUP, TABLE, EXACT, STACK><<<(unsigned)grid, kRefWarps * 32, 0, st>>>(
         px, py, pz, R, theta_sq, force, root_idx, root_node, off, count, stats, max_stack, status);
     return launch_status();
 }
 
-template <typename T, bool TABLE, bool EXACT>
+template <typename T, bool TABLE, bool EXACT, int STACK = 512>
 static int forces_walk(const float *px, const float *py, const float *pz, const RefTree<T> &R,
                        double theta_sq, float *force, const int32_t *root_idx, int32_t root_node,
                        int64_t off, int64_t count, unsigned long long *stats, int32_t *max_stack,
                        int32_t *status, cudaStream_t st) {
     const auto go = [&](auto group) {
-        return launch_walk<T, decltype(group)::value, TABLE, EXACT>(
+        return launch_walk<T, decltype(group)::value, TABLE, EXACT, STACK>(
             px, py, pz, R, theta_sq, force, root_idx, root_node, off, count, stats, max_stack, status, st);
     };
     // A smaller group shares less (more node fetches and tests in all) but gives more warps, and
@@ -412,8 +422,9 @@ int launch_exact_walk(const GroupedParams &P, cudaStream_t st) {
     R.soft2 = normal_soft2(P.soft2);
     R.box = P.box;
     R.m_nodes = P.m_nodes;
-    return forces_walk<float, true, true>(P.px, P.py, P.pz, R, P.theta_sq, P.force, nullptr, P.root, 0,
-                                          P.n, P.stats, P.ws + 2, P.status, st);
+    const auto walk = P.theta < 0.4f ? forces_walk<float, true, true, 848> : forces_walk<float, true, true>;
+    return walk(P.px, P.py, P.pz, R, P.theta_sq, P.force, nullptr, P.root, 0, P.n, P.stats, P.ws + 2, P.status,
+                st);
 }
 
 template <typename T, bool TABLE>

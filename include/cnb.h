@@ -358,8 +358,10 @@ int cnb_exact_test_spill(int every);
 /* With CNB_MAC_REF_X and one theta for all buckets systems of at most this many
  * bodies are walked by groups of consecutive bodies instead of buckets: the
  * same nodes, and faster there than either bucket form.  cnb_forces_two_level
- * makes its lists there too, but walks without them: call cnb_forces_grouped. */
+ * makes its lists there too, but walks without them: call cnb_forces_grouped.
+ * The second limit is for theta below 0.4. */
 #define CNB_EXACT_WALK_BODIES 98304
+#define CNB_EXACT_WALK_BODIES_SMALL_ANGLE 24576
 
 /* Two-level form of cnb_forces_grouped (no reference counterpart; same
  * results as the one-level walk with the same mac, CNB_MAC_REF_X or
