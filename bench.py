@@ -58,7 +58,7 @@ E2E_MIN_STEPS = 40         # steps of the end-to-end measurement (at least --ste
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one force-kernel launch on
 # the 128^3 seed-1 workload at theta 0.5 (64-body buckets, two-level walk with 512-body
 # super-buckets), from one ncu capture of each kernel; not measured by this run
-FORCES_TRAFFIC_BYTES_128 = {"ref_x": 202.8e6 + 21.2e6, "ref_x_bucket": 213.2e6 + 21.8e6}
+FORCES_TRAFFIC_BYTES_128 = {"ref_x": 203.6e6 + 20.9e6, "ref_x_bucket": 213.2e6 + 21.8e6}
 FORCES_KERNEL = {"ref_x": "k_forces_exact", "ref_x_bucket": "k_forces_grouped",
                  "periodic": "k_forces_grouped", "ewald": "k_forces_grouped"}
 
@@ -611,8 +611,8 @@ def run_ours(args):
         achieved = interactions_per_step * FLOPS_PER_INTERACTION / (forces_ms * 1e-3) / 1e12
         traffic = FORCES_TRAFFIC_BYTES_128.get(args.mac) if (
             args.n_grid == 128 and abs(args.theta - 0.5) < 1e-9 and args.force_mode == "grouped") else None
-        line["roofline"] = {"kernel": FORCES_KERNEL.get(args.mac, "k_forces_ref")
-                            if args.force_mode == "grouped" else "k_forces_ref",
+        per_body = args.force_mode != "grouped" or eng.walks_by_groups()
+        line["roofline"] = {"kernel": "k_forces_walk" if per_body else FORCES_KERNEL[args.mac],
                             "bound": "fp32", "achieved": achieved,
                             "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                             "traffic": traffic,

@@ -68,7 +68,9 @@ static_assert(kSplatSlots >= 2 * kSplatThreads * kSplatItems, "a free slot is al
 // exact as a block-wide tile of the grid does, and unlike that they need no
 // bounding box, no passes over its dark pixels, and work for blocks whose
 // pixels are far apart.
-// Bound by the shared-memory atomics.  With the clear (us, a tile of the grid per
+// Bound by the latency of the shared-memory atomics (half of the shared wavefronts;
+// short scoreboard 4.8 stall cycles an issue, the most of any reason; issue 53 %,
+// DRAM 11 %).  With the clear (us, a tile of the grid per
 // block / one global atomic a particle / this): 2M particles on 1920x1080 41 /
 // 18 / 31, 4M on 640x360 56 / 34 / 44, 300 007 on 1024x1024 23 / 8 / 16, 2M on
 // 32x32 106 / 101 / 41, on 4x4 192 / 123 / 31.  The atomics a particle lose
