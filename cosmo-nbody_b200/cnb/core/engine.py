@@ -93,9 +93,15 @@ class SimulationEngine:
         if self.force_mode == "grouped":
             self.set_super_bodies(int(getattr(config, "SUPER_BODIES", 0)))
         self.precision = _lib.PREC_F64 if getattr(config, "PRECISION", "f32") == "f64" else _lib.PREC_F32
-        # reference mode: the node records the per-body walk reads
-        self.ref_table = (torch.empty((4, self.tree_manager.n_nodes, 4), dtype=torch.float32,
-                                      device=state.device) if self.force_mode == "reference" else None)
+        # reference mode: the node records the per-body walk reads, 64 bytes a node; a system
+        # that leaves no room for them is walked over the tree's own arrays
+        self.ref_table = None
+        if self.force_mode == "reference":
+            try:
+                self.ref_table = torch.empty((4, self.tree_manager.n_nodes, 4), dtype=torch.float32,
+                                             device=state.device)
+            except torch.cuda.OutOfMemoryError:
+                pass
         self.stage_events = None
         self.nvtx = False          # NVTX ranges around the step's stages (for nsys / ncu timelines)
         self._nvtx_open = False
@@ -191,6 +197,12 @@ class SimulationEngine:
                       float(cfg.THETA), tpg.data_ptr() if tpg is not None else None, self.mac,
                       self.bodies_per_lane, self.block_warps, float(cfg.G), float(cfg.SOFTENING),
                       float(cfg.BOX_SIZE), self.slab_mass, self.stats.data_ptr(), status, st)
+        elif self.ref_table is None:
+            _lib.call("cnb_compute_forces", px.data_ptr(), py.data_ptr(), pz.data_ptr(),
+                      tm.child.data_ptr(), tm.mass.data_ptr(), tm.com.data_ptr(),
+                      tm.aabb_min.data_ptr(), tm.aabb_max.data_ptr(), s.force.data_ptr(),
+                      float(cfg.THETA), float(cfg.G), float(cfg.SOFTENING), float(cfg.BOX_SIZE),
+                      tm.root_idx.data_ptr(), 0, s.n, s.n, self.precision, status, st)
         else:
             # the nodes once as 32-byte records, then the walk over them
             _lib.call("cnb_pack_nodes", tm.mass.data_ptr(), tm.com.data_ptr(), tm.aabb_min.data_ptr(),
